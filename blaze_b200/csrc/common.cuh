@@ -133,17 +133,16 @@ __device__ __forceinline__ uint32_t lattice_seed(float x, float y, float z, floa
     return lattice_hash(__float2uint_rz(acc));
 }
 
+// One of the library's sixteen gradients: a sum or difference of two
+// of the coordinates.  Selected without branches (the hash differs from lane
+// to lane): bit 0 of h negates the first term, bit 1 the second, which is the
+// library's table exactly, x - y being RN(x + (-y)).
 __device__ __forceinline__ float lattice_grad(int h, float x, float y, float z) {
-    switch (h & 0xF) {
-    case 0x0: return __fadd_rn(x, y);   case 0x1: return __fadd_rn(-x, y);
-    case 0x2: return __fsub_rn(x, y);   case 0x3: return __fsub_rn(-x, y);
-    case 0x4: return __fadd_rn(x, z);   case 0x5: return __fadd_rn(-x, z);
-    case 0x6: return __fsub_rn(x, z);   case 0x7: return __fsub_rn(-x, z);
-    case 0x8: return __fadd_rn(y, z);   case 0x9: return __fadd_rn(-y, z);
-    case 0xA: return __fsub_rn(y, z);   case 0xB: return __fsub_rn(-y, z);
-    case 0xC: return __fadd_rn(y, x);   case 0xD: return __fadd_rn(-y, z);
-    case 0xE: return __fsub_rn(y, x);   default:  return __fsub_rn(-y, z);
-    }
+    h &= 0xF;
+    const float a = h < 8 ? x : y;
+    const float b = h < 4 ? y : (h == 12 || h == 14) ? x : z;
+    return __fadd_rn(__int_as_float(__float_as_int(a) ^ (h << 31)),
+                     __int_as_float(__float_as_int(b) ^ ((h >> 1) << 31)));
 }
 
 // fade (204-207): t^3 (t (6t - 15) + 10), the inner polynomial fused.

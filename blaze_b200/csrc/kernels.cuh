@@ -48,19 +48,21 @@ void launch_splat_gather(const Geom &g, const float *rec8, const int *boxes, con
 
 // -- forces -------------------------------------------------------------------
 void launch_scale(float *a, size_t n, float s, cudaStream_t st);
-void launch_vort_omega(const Geom &g, const float *U, const float *V, const float *W, float *ox,
-                       float *oy, float *oz, cudaStream_t st);
-void launch_vort_force(const Geom &g, const float *U, const float *V, const float *W,
-                       const float *ox, const float *oy, const float *oz, const ForceParams &fp,
-                       float *fx, float *fy, float *fz, cudaStream_t st);
-void launch_face_forces(const Geom &g, float *U, float *V, float *W, const float *T,
-                        const float *fx, const float *fy, const float *fz, const ForceParams &fp,
+// T cooled in place (cool != 1); |omega| (mag) of cells 1..n-2 and omega clamped
+// to the local speed (wx, wy, wz) of cells 2..n-3, of the velocities times drag.
+void launch_vorticity(const Geom &g, float *T, const float *U, const float *V, const float *W, float cool, float drag,
+                      const ForceParams &fp, float *mag, float *wx, float *wy, float *wz, cudaStream_t st);
+// The velocities times drag, confinement (fp.vort_on), buoyancy and wind.
+void launch_face_forces(const Geom &g, float *U, float *V, float *W, const float *T, const float *mag,
+                        const float *wx, const float *wy, const float *wz, const ForceParams &fp, float drag,
                         cudaStream_t st, const float *Dn = nullptr);
 void launch_turb_noise(const Geom &g, const float *T, const float *U, const float *V,
                        const float *W, float *nU, float *nV, float *nW, const ForceParams &fp,
                        cudaStream_t st);
-void launch_turb_apply(const Geom &g, float *U, float *V, float *W, const float *nU,
-                       const float *nV, const float *nW, const ForceParams &fp, cudaStream_t st);
+// Adds the noise's pseudo-curl to the velocities (cx, cy, cz: scratch of T's
+// size; 2 launches).
+void launch_turb_apply(const Geom &g, float *U, float *V, float *W, const float *nU, const float *nV, const float *nW,
+                       const ForceParams &fp, float *cx, float *cy, float *cz, cudaStream_t st);
 
 // cuTensorMapEncodeTiled, looked up once through the runtime's driver entry
 // point (nullptr when the driver has none).

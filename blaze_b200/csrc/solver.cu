@@ -467,31 +467,32 @@ int blz_forces(blz_solver *s, float time) {
     const int c = s->cur, b = c ^ 1;
     float *T = s->T[c], *U = s->U[c], *V = s->V[c], *W = s->W[c];
     const size_t nT = n_of(P, 0);
-    if (std::fabs(P.cooling_rate) > 0.0f) {                                     // FluidSolver.cu:868-872
-        launch_scale(T, nT, 1.0f - P.dt * P.cooling_rate, s->st); CKL(s); s->launches++;
-    }
-    if (P.drag > 0.0f) {                                                        // FluidSolver.cu:878-882
-        const float k = 1.0f - P.dt * P.drag;
-        launch_scale(U, n_of(P, 1), k, s->st); CKL(s);
-        launch_scale(V, n_of(P, 2), k, s->st); CKL(s);
-        launch_scale(W, n_of(P, 3), k, s->st); CKL(s);
+    const ForceParams fp = force_params(s, time);
+    // Cooling and drag (FluidSolver.cu:868-882) ride on the vorticity and face
+    // passes where those run.
+    const bool faces = fp.vort_on || fp.buoy_on || fp.wind_on;
+    const float cool = std::fabs(P.cooling_rate) > 0.0f ? 1.0f - P.dt * P.cooling_rate : 1.0f;
+    const float drag = P.drag > 0.0f ? 1.0f - P.dt * P.drag : 1.0f;
+    if (cool != 1.0f && !fp.vort_on) { launch_scale(T, nT, cool, s->st); CKL(s); s->launches++; }
+    if (drag != 1.0f && !faces) {
+        launch_scale(U, n_of(P, 1), drag, s->st); CKL(s);
+        launch_scale(V, n_of(P, 2), drag, s->st); CKL(s);
+        launch_scale(W, n_of(P, 3), drag, s->st); CKL(s);
         s->launches += 3;
     }
-    const ForceParams fp = force_params(s, time);
-    float *om = s->scratch, *vf = s->scratch + 3 * nT;
+    float *mag = s->scratch, *om = s->scratch + nT;
     if (fp.vort_on) {
-        launch_vort_omega(g, U, V, W, om, om + nT, om + 2 * nT, s->st); CKL(s);
-        launch_vort_force(g, U, V, W, om, om + nT, om + 2 * nT, fp, vf, vf + nT, vf + 2 * nT, s->st); CKL(s);
-        s->launches += 2;
+        launch_vorticity(g, T, U, V, W, cool, drag, fp, mag, om, om + nT, om + 2 * nT, s->st); CKL(s);
+        s->launches++;
     }
-    if (fp.vort_on || fp.buoy_on || fp.wind_on) {
-        launch_face_forces(g, U, V, W, T, vf, vf + nT, vf + 2 * nT, fp, s->st, s->Dn[c]); CKL(s);
+    if (faces) {
+        launch_face_forces(g, U, V, W, T, mag, om, om + nT, om + 2 * nT, fp, drag, s->st, s->Dn[c]); CKL(s);
         s->launches++;
     }
     if (P.turbulence_amp > 0.0f) {                                              // FluidSolver.cu:925-934
         launch_turb_noise(g, T, U, V, W, s->U[b], s->V[b], s->W[b], fp, s->st); CKL(s);
-        launch_turb_apply(g, U, V, W, s->U[b], s->V[b], s->W[b], fp, s->st); CKL(s);
-        s->launches += 2;
+        launch_turb_apply(g, U, V, W, s->U[b], s->V[b], s->W[b], fp, om, om + nT, om + 2 * nT, s->st); CKL(s);
+        s->launches += 3;
     }
     return BLZ_OK;
 }
