@@ -83,6 +83,17 @@ void launch_divergence(const Geom &g, const float *U, const float *V, const floa
 constexpr int kSegVariants = 6;
 constexpr int kSweepVariants = 11;
 int  sweep_variant_count(const Geom &g);
+// The variant after those: the grid kept on chip for the whole batch of
+// sweeps (k_resident.cu), for grids that fit (resident_supported).  `work`:
+// resident_bytes(g) bytes of device memory, zeroed once and kept by the caller
+// for launches ordered on one stream; `err`: mapped host memory, set nonzero
+// when a wait between CTAs gave up (the result is then wrong).
+constexpr int kResidentVariant = kSweepVariants;
+struct ResidentWork { void *work = nullptr; int *err = nullptr; };
+bool resident_supported(const Geom &g);
+size_t resident_bytes(const Geom &g);
+cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
+                            float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st);
 // The temporal-blocking variant whose loads are TMA bulk copies (bounded
 // waits that may give up: tb_take_timeouts).
 bool sweep_variant_uses_tma(int v);
@@ -91,7 +102,8 @@ bool sweep_variant_uses_tma(int v);
 unsigned int tb_take_timeouts();
 void launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r,
                         const float *rhs_b, float *p_r, float *p_b, int sweeps, cudaStream_t st,
-                        long long *launches, int variant = 0, float *q_r = nullptr, float *q_b = nullptr);
+                        long long *launches, int variant = 0, float *q_r = nullptr, float *q_b = nullptr,
+                        const ResidentWork &res = {});
 // The pressure system solved in FP64 (SOR, natural layout) to relative
 // residual tol, the result rounded into p (tight.cu).  Returns 0 or a
 // cudaError_t.
@@ -160,7 +172,8 @@ cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float 
                               float *p_r, float *p_b, double *partials, int n_partials, double *norm2,
                               SolveCtl *ctl, int chunk, int max_iter, double tol, int variant, cudaStream_t st,
                               cudaGraphExec_t *exec_out, int *body_kernels, int *prologue_kernels,
-                              float *q_r = nullptr, float *q_b = nullptr, const DefectArrays *dfa = nullptr);
+                              float *q_r = nullptr, float *q_b = nullptr, const DefectArrays *dfa = nullptr,
+                              const ResidentWork &res = {});
 
 // -- batched solve over many grids (k_project.cu kernels, batch.cu graph) ---
 struct BatchSim {

@@ -58,6 +58,7 @@ struct blz_solver {
     long long launches = 0;
     blz_unet *warm = nullptr;                   // learned warm start (caller owned)
     int variant = -2;                           // sweep launch shape (-2: not chosen yet)
+    ResidentWork res;                           // on-chip sweeps: exchange buffers, error flag
     // device-loop solve: instantiated graphs (one per check interval used)
     // and their control block
     struct SolveGraph {
@@ -185,6 +186,7 @@ static void release(blz_solver *s) {
     for (auto &gr : s->graphs)
         if (gr.exec) cudaGraphExecDestroy(gr.exec);
     cudaFree(s->ctl);
+    cudaFree(s->res.work);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
     for (auto &e : s->ev) if (e) cudaEventDestroy(e);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);
@@ -257,9 +259,15 @@ int blz_create(const blz_params *p, blz_solver **out) {
     s->n_partials = residual_blocks(g);
     ok = ok && cudaMalloc(&s->partials, 2 * sizeof(double) * s->n_partials) == cudaSuccess;
     ok = ok && cudaMalloc(&s->d_norm2, 2 * sizeof(double)) == cudaSuccess;
-    ok = ok && cudaMallocHost(&s->h_norm2, 2 * sizeof(double)) == cudaSuccess;
+    ok = ok && cudaMallocHost(&s->h_norm2, 4 * sizeof(double)) == cudaSuccess;   // two norms; the on-chip sweeps' error flag
     ok = ok && cudaMalloc(&s->ctl, sizeof(SolveCtl)) == cudaSuccess;
     ok = ok && cudaMallocHost(&s->h_ctl, sizeof(SolveCtl)) == cudaSuccess;
+    if (ok && p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 && resident_supported(g)) {
+        ok = cudaMalloc(&s->res.work, resident_bytes(g)) == cudaSuccess &&
+             cudaMemset(s->res.work, 0, resident_bytes(g)) == cudaSuccess;
+        s->res.err = reinterpret_cast<int *>(s->h_norm2 + 2);
+        if (ok) *s->res.err = 0;
+    }
     if (!ok) { cudaGetLastError(); int r = fail(s, BLZ_ERR_ALLOC, "device allocation failed for %dx%dx%d", g.W, g.H, g.D); return bail(r); }
     for (auto &ev : s->ev)
         if (cudaEventCreate(&ev) != cudaSuccess) { int r = fail(s, BLZ_ERR_CUDA, "cudaEventCreate failed"); return bail(r); }
@@ -572,7 +580,7 @@ static std::map<std::tuple<int, int, int, int>, int> g_tune_cache;
 
 // The tuner's choices persist across processes in a small text file, one
 // line "<device name>|<W>|<H>|<D>|<variants offered>|<variant count> <choice>"
-// per grid: BLZ_TUNE_CACHE names the file ("off" or empty: none), default
+// per grid ("+on-chip" after the name where the on-chip sweeps are offered too): BLZ_TUNE_CACHE names the file ("off" or empty: none), default
 // $XDG_CACHE_HOME/blaze_b200/sweep_variants.txt or ~/.cache/... .
 static std::string tune_cache_path() {
     if (const char *p = std::getenv("BLZ_TUNE_CACHE")) {
@@ -586,11 +594,11 @@ static std::string tune_cache_path() {
     return base + "/blaze_b200/sweep_variants.txt";
 }
 
-static std::string tune_key(int device, const Geom &g, int offered) {
+static std::string tune_key(int device, const Geom &g, int offered, bool on_chip) {
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) return std::string();
     char buf[400];
-    std::snprintf(buf, sizeof buf, "%s|%d|%d|%d|%d|%d", prop.name, g.W, g.H, g.D, offered, kSweepVariants);
+    std::snprintf(buf, sizeof buf, "%s%s|%d|%d|%d|%d|%d", prop.name, on_chip ? "+on-chip" : "", g.W, g.H, g.D, offered, kSweepVariants);
     for (char *c = buf; *c; ++c)
         if (*c == ' ') *c = '_';
     return buf;
@@ -632,19 +640,26 @@ static int choose_variant(blz_solver *s) {
     const int nv = s->P.temporal_block == 1 ? std::min(sweep_variant_count(s->g), kSegVariants)
                                             : sweep_variant_count(s->g);
     if (nv == 0) { s->variant = -1; return BLZ_OK; }
-    if (s->P.sweep_variant >= 0) { s->variant = std::min(s->P.sweep_variant, nv - 1); return BLZ_OK; }
-    if (const char *env = std::getenv("BLZ_SWEEP_VARIANT")) {
-        s->variant = std::max(0, std::min(std::atoi(env), nv - 1));
-        return BLZ_OK;
-    }
+    // A forced choice; the on-chip sweeps (past the launch shapes) only where
+    // the grid fits.
+    auto forced = [&](int v) { return v == kResidentVariant && s->res.work ? v : std::max(0, std::min(v, nv - 1)); };
+    if (s->P.sweep_variant >= 0) { s->variant = forced(s->P.sweep_variant); return BLZ_OK; }
+    if (const char *env = std::getenv("BLZ_SWEEP_VARIANT")) { s->variant = forced(std::atoi(env)); return BLZ_OK; }
+    // Candidates: every launch shape, or, for a grid that fits on chip, the on-
+    // chip sweeps and the two shapes nearest to them (1.6 to 4.0 us per sweep
+    // from 32^3 to 128^3 against 3.8 to 6.7; the temporal-blocking passes take
+    // 8 us and more there), so that the first solve of a grid times three.
+    std::vector<int> cand;
+    if (s->res.work) cand = {0, 4, kResidentVariant};
+    else for (int v = 0; v < nv; ++v) cand.push_back(v);
     const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D * 2 + (nv > kSegVariants ? 1 : 0));
-    const std::string fkey = tune_key(s->device, s->g, nv);
+    const std::string fkey = tune_key(s->device, s->g, nv, s->res.work != nullptr);
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) { s->variant = it->second; return BLZ_OK; }
         const int v = tune_file_lookup(fkey);
-        if (v >= 0 && v < nv) {
+        if ((v >= 0 && v < nv) || (v == kResidentVariant && s->res.work)) {
             g_tune_cache[key] = v;
             s->variant = v;
             return BLZ_OK;
@@ -658,8 +673,8 @@ static int choose_variant(blz_solver *s) {
     long long dummy = 0;
     // Direct launches first: they set the kernels' attributes outside any
     // capture and warm the SM clock.
-    for (int v = 0; v < nv; ++v)
-        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, 4, s->st, &dummy, v, q_r(s), q_b(s));
+    for (int v : cand)
+        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, 4, s->st, &dummy, v, q_r(s), q_b(s), s->res);
     CKL(s);
     CK(s, cudaStreamSynchronize(s->st));
     // Each variant is timed as the solve runs it: kTuneSweeps sweeps (one
@@ -670,27 +685,28 @@ static int choose_variant(blz_solver *s) {
     constexpr int kTuneSweeps = 20;
     cudaStream_t ts = nullptr;
     CK(s, cudaStreamCreateWithFlags(&ts, cudaStreamNonBlocking));
-    std::vector<cudaGraphExec_t> ex(nv, nullptr);
-    std::vector<long long> per_graph(nv, 0);
-    std::vector<float> t_min(nv, 1e30f);
+    const int nc = (int)cand.size();
+    std::vector<cudaGraphExec_t> ex(nc, nullptr);
+    std::vector<long long> per_graph(nc, 0);
+    std::vector<float> t_min(nc, 1e30f);
     cudaError_t err = cudaSuccess;
-    for (int v = 0; v < nv && err == cudaSuccess; ++v) {
+    for (int v = 0; v < nc && err == cudaSuccess; ++v) {
         cudaGraph_t gph = nullptr;
         err = cudaStreamBeginCapture(ts, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
-        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, kTuneSweeps, ts, &per_graph[v], v, q_r(s),
-                           q_b(s));
+        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, kTuneSweeps, ts, &per_graph[v], cand[v], q_r(s),
+                           q_b(s), s->res);
         err = cudaStreamEndCapture(ts, &gph);
         if (err == cudaSuccess) err = cudaGraphInstantiate(&ex[v], gph, 0);
         if (gph) cudaGraphDestroy(gph);
     }
-    for (int v = 0; v < nv && err == cudaSuccess; ++v) {
+    for (int v = 0; v < nc && err == cudaSuccess; ++v) {
         err = cudaGraphLaunch(ex[v], ts);
         if (err == cudaSuccess) dummy += per_graph[v];
     }
     for (int round = 0; round < 2 && err == cudaSuccess; ++round)
-        for (int i = 0; i < nv && err == cudaSuccess; ++i) {
-            const int v = round == 0 ? i : nv - 1 - i;
+        for (int i = 0; i < nc && err == cudaSuccess; ++i) {
+            const int v = round == 0 ? i : nc - 1 - i;
             float ms = 0.0f;
             err = cudaEventRecord(s->ev[6], ts);
             if (err == cudaSuccess) err = cudaGraphLaunch(ex[v], ts);
@@ -705,10 +721,10 @@ static int choose_variant(blz_solver *s) {
         if (e) cudaGraphExecDestroy(e);
     cudaStreamDestroy(ts);
     if (err != cudaSuccess) return fail(s, BLZ_ERR_CUDA, "sweep autotuner: %s", cudaGetErrorString(err));
-    const int best = (int)(std::min_element(t_min.begin(), t_min.end()) - t_min.begin());
+    const int best = cand[std::min_element(t_min.begin(), t_min.end()) - t_min.begin()];
     if (std::getenv("BLZ_TUNE_VERBOSE")) {
         std::fprintf(stderr, "sweep autotuner %dx%dx%d, us per sweep:", s->g.W, s->g.H, s->g.D);
-        for (int v = 0; v < nv; ++v) std::fprintf(stderr, " v%d=%.2f", v, 1e3f * t_min[v] / kTuneSweeps);
+        for (int v = 0; v < nc; ++v) std::fprintf(stderr, " v%d=%.2f", cand[v], 1e3f * t_min[v] / kTuneSweeps);
         std::fprintf(stderr, " -> v%d\n", best);
     }
     s->launches += dummy;
@@ -726,7 +742,7 @@ static int sweeps_on(blz_solver *s, int n, const float *rr, const float *rb, flo
     } else {
         int rc = choose_variant(s);
         if (rc != BLZ_OK) return rc;
-        launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, s->variant, q_r(s), q_b(s));
+        launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, s->variant, q_r(s), q_b(s), s->res);
     }
     CKL(s);
     return BLZ_OK;
@@ -775,7 +791,7 @@ static int solve_device_loop(blz_solver *s, blz_step_stats *st, int chunk) {
         cudaError_t e = build_solve_graph(s->g, solve_params(P), s->sr_r, s->sr_b, s->sx_r, s->sx_b, s->partials,
                                           s->n_partials, s->d_norm2, s->ctl, chunk, P.max_iter, P.tol, s->variant,
                                           s->st, &gr->exec, &gr->body, &gr->prologue, q_r(s), q_b(s),
-                                          P.defect_correction ? &dfa : nullptr);
+                                          P.defect_correction ? &dfa : nullptr, s->res);
         if (e != cudaSuccess) return fail(s, BLZ_ERR_CUDA, "building the solve graph failed: %s", cudaGetErrorString(e));
         gr->chunk = chunk;
     }
@@ -807,9 +823,18 @@ static int solve_device_loop(blz_solver *s, blz_step_stats *st, int chunk) {
 
 static int solve_body(blz_solver *s, blz_step_stats *st);
 
-// The TMA-staged pass counts bounded waits that gave up; after work that may
-// have used it, a nonzero count is reported (that pass's result is wrong).
+// The TMA-staged pass counts bounded waits that gave up, the on-chip sweeps flag
+// them; after work that may have used either, they are reported (the result is
+// wrong).  The flag is in host memory: no synchronisation to read it, and a
+// failure of sweeps still in flight shows at the next call that looks.
+static int take_resident_error(blz_solver *s) {
+    if (!s->res.err || !*(volatile int *)s->res.err) return BLZ_OK;
+    *(volatile int *)s->res.err = 0;
+    return fail(s, BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up");
+}
+
 static int check_tb_timeouts(blz_solver *s) {
+    if (s->variant == kResidentVariant) return take_resident_error(s);
     if (!sweep_variant_uses_tma(s->variant)) return BLZ_OK;
     CK(s, cudaStreamSynchronize(s->st));
     if (tb_take_timeouts()) return fail(s, BLZ_ERR_TIMEOUT, "temporal-blocking pass: a bounded TMA wait gave up");
@@ -837,7 +862,7 @@ static int warm_start(blz_solver *s, int variant, int *pre) {
                                &s->launches, variant, q_r(s), q_b(s));
         }
         launch_rbgs_sweeps(s->g, solve_params(P), z_r, z_b, d_r, d_b, *pre, s->st, &s->launches, variant, q_r(s),
-                           q_b(s));
+                           q_b(s), s->res);
         CKL(s);
     } else {
         *pre = 0;
@@ -1107,7 +1132,7 @@ int blz_get_field(blz_solver *s, int f, float *dst, int on_device) {
     }
     CK(s, cudaMemcpyAsync(dst, src, n * sizeof(float), kind, s->st));
     CK(s, cudaStreamSynchronize(s->st));
-    return BLZ_OK;
+    return take_resident_error(s);
 }
 
 int blz_set_field(blz_solver *s, int f, const float *src, int on_device) {
