@@ -895,11 +895,15 @@ void launch_plane_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_
 constexpr int kResThreads = 256;
 
 // Tiles of the z-marching residual (W % 8 == 0 and W <= 2048): a block of
-// kResThreads threads covers kResThreads / Wq rows of quads and kResKZ planes.
-// 16 planes and at most 64 registers (four blocks per SM): at 256^3 the 512
-// tiles are one wave, with 32 warps per SM waiting on DRAM.
+// kResThreads threads covers kResThreads / Wq rows of quads and residual_kz(g)
+// planes.  At most 64 registers (four blocks per SM): at 256^3 the 512 tiles of
+// 16 planes are one wave, with 32 warps per SM waiting on DRAM.  A smaller grid
+// halves the planes (a divisor of the slabs' 16) until it has as many tiles:
+// its residual is bound by the chain of planes of one tile, 25 us at 64^3 with
+// 16 planes in 8 blocks, 6.6 us with 2.
 constexpr int kResKZ = 16;
 constexpr int kResBlocksPerSM = 4;
+constexpr int kResTilesWanted = 512;
 
 __host__ __device__ inline bool residual_tiled(const Geom &g) { return (g.W & 7) == 0 && (g.W >> 3) <= kResThreads; }
 __host__ __device__ inline int residual_tile_rows(const Geom &g) { return kResThreads / (g.W >> 3); }
@@ -907,9 +911,15 @@ __host__ __device__ inline int residual_tiles_y(const Geom &g) {
     const int R = residual_tile_rows(g);
     return (g.H + R - 1) / R;
 }
+__host__ __device__ inline int residual_kz(const Geom &g) {
+    int kz = kResKZ;
+    while (kz > 2 && residual_tiles_y(g) * ((g.D + kz - 1) / kz) < kResTilesWanted) kz >>= 1;
+    return kz;
+}
 
 __host__ __device__ inline int residual_tiles(const Geom &g) {
-    return residual_tiles_y(g) * ((g.D + kResKZ - 1) / kResKZ);
+    const int kz = residual_kz(g);
+    return residual_tiles_y(g) * ((g.D + kz - 1) / kz);
 }
 
 // Partial sums one residual of g produces: one per tile, else one per block.
@@ -1035,7 +1045,7 @@ __device__ __forceinline__ void block_pair_sum(double r2, double b2, double *__r
 }
 
 // Tile `blk` of the z-marching residual: each thread takes one quad of a row
-// through kResKZ planes, carrying both colours' quads of planes k-1, k, k+1
+// through residual_kz(g) planes, carrying both colours' quads of planes k-1, k, k+1
 // in registers (one new plane of each per step), red cells then black cells
 // per plane; the block's FP64 sums go to partials[2*blk], [2*blk + 1].
 __device__ __forceinline__ void residual_tile_block(const Geom &g, const SolveParams &sp, double scale,
@@ -1043,10 +1053,10 @@ __device__ __forceinline__ void residual_tile_block(const Geom &g, const SolvePa
                                                     const float *__restrict__ pr, const float *__restrict__ pb,
                                                     int blk, double *__restrict__ partials) {
     const int Wh = g.W >> 1, Wq = Wh >> 2;
-    const int R = residual_tile_rows(g), ty = residual_tiles_y(g);
+    const int R = residual_tile_rows(g), ty = residual_tiles_y(g), kz = residual_kz(g);
     const int t = threadIdx.x;
     const int mq = t % Wq, jr = t / Wq;
-    const int j = (blk % ty) * R + jr, k0 = (blk / ty) * kResKZ;
+    const int j = (blk % ty) * R + jr, k0 = (blk / ty) * kz;
     double r2 = 0.0, b2 = 0.0;
     if (jr < R && j < g.H) {
         const size_t pl = (size_t)Wh * g.H;
@@ -1056,7 +1066,7 @@ __device__ __forceinline__ void residual_tile_block(const Geom &g, const SolvePa
         const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
         float4 rm = k0 > 0 ? ld4(pr + row + (k0 - 1) * pl) : zero4, bm = k0 > 0 ? ld4(pb + row + (k0 - 1) * pl) : zero4;
         float4 rc = ld4(pr + row + k0 * pl), bc = ld4(pb + row + k0 * pl);
-        const int k1 = k0 + kResKZ < g.D ? k0 + kResKZ : g.D;
+        const int k1 = k0 + kz < g.D ? k0 + kz : g.D;
         for (int k = k0; k < k1; ++k) {
             const size_t q = row + (size_t)k * pl;
             const bool has_zm = k > 0, has_zp = k < g.D - 1;
@@ -1086,11 +1096,27 @@ __device__ __forceinline__ void residual_block(const Geom &g, const SolveParams 
     else residual_seg_block(g, sp, scale, rr, rb, pr, pb, blk, nblk, partials);
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The first kernel of a device-loop check ends the sweep interval and starts
+// the check interval (c null outside one).
+__device__ __forceinline__ void mark_check(SolveCtl *c) {
+    if (!c || blockIdx.x != 0 || threadIdx.x != 0) return;
+    const unsigned long long t = global_ns();
+    c->sweep_ns += t - c->t0;
+    c->t1 = t;
+}
+
 // One block per tile when residual_tiled(g), else grid-stride segments.
 __global__ void __launch_bounds__(kResThreads, kResBlocksPerSM)
 k_residual_seg(Geom g, SolveParams sp, double scale, const float *__restrict__ rr,
                const float *__restrict__ rb, const float *__restrict__ pr, const float *__restrict__ pb,
-               double *__restrict__ partials) {
+               double *__restrict__ partials, SolveCtl *ctl) {
+    mark_check(ctl);
     residual_block(g, sp, scale, rr, rb, pr, pb, blockIdx.x, gridDim.x, partials);
 }
 
@@ -1098,7 +1124,8 @@ k_residual_seg(Geom g, SolveParams sp, double scale, const float *__restrict__ r
 __global__ void __launch_bounds__(kResThreads)
 k_residual(Geom g, SolveParams sp, double scale, const float *__restrict__ rr,
            const float *__restrict__ rb, const float *__restrict__ pr, const float *__restrict__ pb,
-           double *__restrict__ partials) {
+           double *__restrict__ partials, SolveCtl *ctl) {
+    mark_check(ctl);
     const int Wh = g.W >> 1;
     const int items = Wh * g.H * g.D;
     double r2 = 0.0, b2 = 0.0;
@@ -1166,18 +1193,55 @@ __global__ void __launch_bounds__(1024) k_reduce_pairs(const double *__restrict_
     reduce_pairs_block(partials, n, out2);
 }
 
+// k_reduce_pairs with the device loop's decision: records {||r||^2, ||b||^2}
+// and the times, sets whether the loop goes on and starts the next sweep
+// interval.  after_sweeps = 0 is the check before any sweep, which also resets
+// the control block.
+__global__ void __launch_bounds__(1024)
+k_reduce_check(const double *__restrict__ partials, int n, double *__restrict__ out2, SolveCtl *c,
+               cudaGraphConditionalHandle h, int after_sweeps, int chunk, int max_iter, double tol) {
+    __shared__ double s2[2];
+    reduce_pairs_block(partials, n, s2);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    const double r2 = s2[0], b2 = s2[1];
+    out2[0] = r2;
+    out2[1] = b2;
+    const int iters = after_sweeps ? c->iters + chunk : 0;
+    const bool conv = b2 == 0.0 || sqrt(r2) / sqrt(b2) <= tol;
+    c->iters = iters;
+    c->checks = after_sweeps ? c->checks + 1 : 1;
+    c->r2 = r2;
+    c->b2 = b2;
+    c->converged = conv;
+    const unsigned long long t = global_ns();
+    if (after_sweeps) c->check_ns += t - c->t1;
+    else c->sweep_ns = c->check_ns = 0;
+    c->t0 = t;
+    cudaGraphSetConditional(h, (!conv && iters < max_iter) ? 1u : 0u);
+}
+
+static void launch_pairs(const double *partials, int n, double *out2, const LoopCheck *loop, cudaStream_t st) {
+    if (loop)
+        k_reduce_check<<<1, 1024, 0, st>>>(partials, n, out2, loop->ctl, loop->handle, loop->after_sweeps, loop->chunk,
+                                           loop->max_iter, loop->tol);
+    else
+        k_reduce_pairs<<<1, 1024, 0, st>>>(partials, n, out2);
+}
+static SolveCtl *check_mark(const LoopCheck *loop) { return loop && loop->after_sweeps ? loop->ctl : nullptr; }
+
 int launch_residual(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b,
                     const float *p_r, const float *p_b, double *partials, int max_partials,
-                    double *out2, cudaStream_t st) {
+                    double *out2, cudaStream_t st, const LoopCheck *loop) {
     // max_partials is residual_blocks(g) (the partials buffer of the solver)
     const int parts = std::min(residual_blocks(g), max_partials);
     const double scale = (double)sp.scale_d;
     if ((g.W & 7) == 0) {
-        k_residual_seg<<<parts, kResThreads, 0, st>>>(g, sp, scale, rhs_r, rhs_b, p_r, p_b, partials);
+        k_residual_seg<<<parts, kResThreads, 0, st>>>(g, sp, scale, rhs_r, rhs_b, p_r, p_b, partials, check_mark(loop));
     } else {
-        k_residual<<<parts, kResThreads, 0, st>>>(g, sp, scale, rhs_r, rhs_b, p_r, p_b, partials);
+        k_residual<<<parts, kResThreads, 0, st>>>(g, sp, scale, rhs_r, rhs_b, p_r, p_b, partials, check_mark(loop));
     }
-    k_reduce_pairs<<<1, 1024, 0, st>>>(partials, parts, out2);
+    launch_pairs(partials, parts, out2, loop, st);
     return 2;
 }
 
@@ -1193,9 +1257,9 @@ k_residual_tiles(Geom g, SolveParams sp, double scale, const float *__restrict__
 int residual_slab_tiles(const Geom &g, int z0, int z1, int *first, int *count) {
     if (!residual_tiled(g) || z0 < 0 || z1 > g.D || z0 >= z1 || z0 % kResKZ != 0 || (z1 % kResKZ != 0 && z1 != g.D))
         return -1;
-    const int ty = residual_tiles_y(g);
-    *first = (z0 / kResKZ) * ty;
-    *count = ((z1 + kResKZ - 1) / kResKZ - z0 / kResKZ) * ty;
+    const int ty = residual_tiles_y(g), kz = residual_kz(g);
+    *first = (z0 / kz) * ty;
+    *count = ((z1 + kz - 1) / kz - z0 / kz) * ty;
     return 0;
 }
 
@@ -1313,7 +1377,7 @@ void launch_gradient(const Geom &g, const SolveParams &sp, float s, const float 
 // for the correction delta) and the residual of the pressure p + delta,
 // r = b - A p - A delta (both stencils in deviation form, exact in FP64).
 // Per-block partial sums of r^2 and b^2 go to part[2 * block] and
-// part[2 * block + 1]; k_defect_total sums them in block order into
+// part[2 * block + 1], summed in k_reduce_pairs' order into
 // out2 = {||r||^2, ||b||^2}.
 constexpr int kDefectThreads = 256;
 constexpr int kDefectBlocks = 1184;
@@ -1331,25 +1395,7 @@ __device__ __forceinline__ double stencil64(const float *__restrict__ pr, const 
     return d;
 }
 
-__global__ void __launch_bounds__(kDefectThreads)
-k_defect(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
-         const float *__restrict__ pr, const float *__restrict__ pb, const float *__restrict__ dr,
-         const float *__restrict__ db, float *__restrict__ def_r, float *__restrict__ def_b,
-         double *__restrict__ part) {
-    const int Wh = g.W >> 1, H = g.H;
-    const long long n = (long long)g.W * g.H * g.D;
-    double r2 = 0.0, b2 = 0.0;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < n; c += (long long)gridDim.x * blockDim.x) {
-        const int i = (int)(c % g.W), j = (int)((c / g.W) % g.H), k = (int)(c / ((long long)g.W * g.H));
-        const size_t q = pidx(i, j, k, Wh, H);
-        const bool black = (i + j + k) & 1;
-        const double b = sp.scale_d * (double)(black ? rhs_b : rhs_r)[q];
-        const double bp = b - stencil64(pr, pb, i, j, k, g.W, g.H, g.D, Wh, sp.open, sp.dirichlet);
-        (black ? def_b : def_r)[q] = (float)(bp / sp.scale_d);
-        const double r = bp - stencil64(dr, db, i, j, k, g.W, g.H, g.D, Wh, sp.open, sp.dirichlet);
-        r2 += r * r;
-        b2 += b * b;
-    }
+__device__ __forceinline__ void defect_sums(double r2, double b2, double *__restrict__ part) {
     __shared__ double sr[kDefectThreads], sb[kDefectThreads];
     sr[threadIdx.x] = r2;
     sb[threadIdx.x] = b2;
@@ -1361,12 +1407,95 @@ k_defect(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *_
     if (threadIdx.x == 0) { part[2 * blockIdx.x] = sr[0]; part[2 * blockIdx.x + 1] = sb[0]; }
 }
 
-__global__ void k_defect_total(const double *__restrict__ part, int nb, double *__restrict__ out2) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// One cell per item: rows of any even width.
+__global__ void __launch_bounds__(kDefectThreads)
+k_defect(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
+         const float *__restrict__ pr, const float *__restrict__ pb, const float *__restrict__ dr,
+         const float *__restrict__ db, float *__restrict__ def_r, float *__restrict__ def_b,
+         double *__restrict__ part) {
+    const int Wh = g.W >> 1, H = g.H, n = g.W * g.H * g.D;
+    const double inv = 1.0 / sp.scale_d;
     double r2 = 0.0, b2 = 0.0;
-    for (int t = 0; t < nb; ++t) { r2 += part[2 * t]; b2 += part[2 * t + 1]; }
-    out2[0] = r2;
-    out2[1] = b2;
+    for (long long t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int c = (int)t, i = c % g.W, jk = c / g.W, j = jk % g.H, k = jk / g.H;
+        const size_t q = pidx(i, j, k, Wh, H);
+        const bool black = (i + j + k) & 1;
+        const double b = sp.scale_d * (double)(black ? rhs_b : rhs_r)[q];
+        const double bp = b - stencil64(pr, pb, i, j, k, g.W, g.H, g.D, Wh, sp.open, sp.dirichlet);
+        (black ? def_b : def_r)[q] = (float)(bp * inv);
+        const double r = bp - stencil64(dr, db, i, j, k, g.W, g.H, g.D, Wh, sp.open, sp.dirichlet);
+        r2 += r * r;
+        b2 += b * b;
+    }
+    defect_sums(r2, b2, part);
+}
+
+// A x of four packed cells of one colour of a row (W % 8 == 0), x the cells'
+// own values, q the packed index of the first, o the other colour; terms in
+// stencil64's order.
+__device__ __forceinline__ void stencil64_quad(const float *__restrict__ x, const float *__restrict__ o, int q, int Wh,
+                                               int pl, int s, bool first, bool last, bool ym, bool yp, bool zm, bool zp,
+                                               const OpenFaces &f, bool dir, double (&out)[4]) {
+    const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 c4 = ld4(x + q), o4 = ld4(o + q);
+    const float xe = s == 0 ? (first ? 0.0f : __ldg(o + q - 1)) : (last ? 0.0f : __ldg(o + q + 4));
+    const float4 y0 = ym ? ld4(o + q - Wh) : zero4, y1 = yp ? ld4(o + q + Wh) : zero4;
+    const float4 z0 = zm ? ld4(o + q - pl) : zero4, z1 = zp ? ld4(o + q + pl) : zero4;
+    const float c[4] = {c4.x, c4.y, c4.z, c4.w};
+    const float row[5] = {s == 0 ? xe : o4.x, s == 0 ? o4.x : o4.y, s == 0 ? o4.y : o4.z, s == 0 ? o4.z : o4.w,
+                          s == 0 ? o4.w : xe};
+    const float ya[4] = {y0.x, y0.y, y0.z, y0.w}, yb[4] = {y1.x, y1.y, y1.z, y1.w};
+    const float za[4] = {z0.x, z0.y, z0.z, z0.w}, zb[4] = {z1.x, z1.y, z1.z, z1.w};
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+        const double pc = (double)c[t];
+        // a missing neighbour: the cell itself (no flow), or 0 at a ghost
+        auto term = [&](bool has, float nb, bool open) { return has ? pc - (double)nb : dir && open ? pc : 0.0; };
+        double d = term(!(s == 0 && first && t == 0), row[t], f.xlo);
+        d += term(!(s == 1 && last && t == 3), row[t + 1], f.xhi);
+        d += term(ym, ya[t], f.ylo);
+        d += term(yp, yb[t], f.yhi);
+        d += term(zm, za[t], f.zlo);
+        d += term(zp, zb[t], f.zhi);
+        out[t] = d;
+    }
+}
+
+// Four packed cells of both colours per item (W % 8 == 0), 128-bit loads and
+// stores; neighbouring rows and planes come from L1 and L2.  Measured at 384^3:
+// 421 us (one cell per item with 64-bit index arithmetic: 1882 us).
+__global__ void __launch_bounds__(kDefectThreads)
+k_defect_quad(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
+              const float *__restrict__ pr, const float *__restrict__ pb, const float *__restrict__ dr,
+              const float *__restrict__ db, float *__restrict__ def_r, float *__restrict__ def_b,
+              double *__restrict__ part) {
+    const int Wh = g.W >> 1, Wq = Wh >> 2, pl = Wh * g.H, n = Wq * g.H * g.D;
+    const double inv = 1.0 / sp.scale_d;
+    double r2 = 0.0, b2 = 0.0;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+        const int mq = t % Wq, jk = t / Wq, j = jk % g.H, k = jk / g.H;
+        const int q = 4 * t;
+        const bool ym = j > 0, yp = j < g.H - 1, zm = k > 0, zp = k < g.D - 1, first = mq == 0, last = mq == Wq - 1;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int s = (j + k + c) & 1;
+            double ap[4], ad[4];
+            stencil64_quad(c ? pb : pr, c ? pr : pb, q, Wh, pl, s, first, last, ym, yp, zm, zp, sp.open, sp.dirichlet, ap);
+            stencil64_quad(c ? db : dr, c ? dr : db, q, Wh, pl, s, first, last, ym, yp, zm, zp, sp.open, sp.dirichlet, ad);
+            const float4 h = ld4((c ? rhs_b : rhs_r) + q);
+            const float rhs[4] = {h.x, h.y, h.z, h.w};
+            float out[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const double b = sp.scale_d * (double)rhs[e], bp = b - ap[e], r = bp - ad[e];
+                out[e] = (float)(bp * inv);
+                r2 += r * r;
+                b2 += b * b;
+            }
+            *reinterpret_cast<float4 *>((c ? def_b : def_r) + q) = make_float4(out[0], out[1], out[2], out[3]);
+        }
+    }
+    defect_sums(r2, b2, part);
 }
 
 // p = RN(p + delta) and delta = (p + delta) - RN(p + delta), exactly (Knuth's
@@ -1380,7 +1509,8 @@ __device__ __forceinline__ void two_sum(float &a, float &b) {
     a = s;
 }
 __global__ void k_fold(long long n, float *__restrict__ pr, float *__restrict__ pb, float *__restrict__ dr,
-                       float *__restrict__ db) {
+                       float *__restrict__ db, SolveCtl *ctl) {
+    mark_check(ctl);
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
         float a = pr[t], b = dr[t];
         two_sum(a, b);
@@ -1396,16 +1526,17 @@ __global__ void k_fold(long long n, float *__restrict__ pr, float *__restrict__ 
 
 int launch_defect(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, const float *p_r,
                   const float *p_b, const float *d_r, const float *d_b, float *def_r, float *def_b, double *partials,
-                  int max_partials, double *out2, cudaStream_t st) {
+                  int max_partials, double *out2, cudaStream_t st, const LoopCheck *loop) {
     const int nb = std::min(kDefectBlocks, max_partials);
-    k_defect<<<nb, kDefectThreads, 0, st>>>(g, sp, rhs_r, rhs_b, p_r, p_b, d_r, d_b, def_r, def_b, partials);
-    k_defect_total<<<1, 32, 0, st>>>(partials, nb, out2);
+    const auto k = (g.W & 7) == 0 ? k_defect_quad : k_defect;
+    k<<<nb, kDefectThreads, 0, st>>>(g, sp, rhs_r, rhs_b, p_r, p_b, d_r, d_b, def_r, def_b, partials);
+    launch_pairs(partials, nb, out2, loop, st);
     return 2;
 }
 
-void launch_fold(const Geom &g, float *p_r, float *p_b, float *d_r, float *d_b, cudaStream_t st) {
+void launch_fold(const Geom &g, float *p_r, float *p_b, float *d_r, float *d_b, cudaStream_t st, const LoopCheck *loop) {
     const long long n = (long long)g.W * g.H * g.D / 2;
-    k_fold<<<(int)std::min<long long>((n + 255) / 256, 4736), 256, 0, st>>>(n, p_r, p_b, d_r, d_b);
+    k_fold<<<(int)std::min<long long>((n + 255) / 256, 4736), 256, 0, st>>>(n, p_r, p_b, d_r, d_b, check_mark(loop));
 }
 
 __global__ void k_pack(Geom g, const float *__restrict__ nat, float *__restrict__ red,

@@ -113,11 +113,27 @@ int tight_solve(const Geom &g, const SolveParams &sp, const float *rhs_r, const 
 void launch_plane_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r,
                          const float *rhs_b, float *p_r, float *p_b, int sweeps, cudaStream_t st,
                          long long *launches);
+// Device-side state of a graph-run solve (see graph_solve.cu).
+struct SolveCtl {
+    int iters, checks, converged, pad;
+    double r2, b2;                      // last ||r||^2, ||b||^2
+    unsigned long long sweep_ns, t0;    // global-timer time inside sweep batches
+    unsigned long long check_ns, t1;    // ... and inside the residual checks
+};
+// A residual check inside the device loop: its last kernel takes the decision
+// and its first ends the sweep interval (graph_solve.cu).  after_sweeps = 0: the
+// check before any sweep.
+struct LoopCheck {
+    SolveCtl *ctl;
+    cudaGraphConditionalHandle handle;
+    int after_sweeps, chunk, max_iter;
+    double tol;
+};
 // Writes partial sums to `partials` (2 doubles per block) and the totals
 // {||r||^2, ||b||^2} to out2.  Returns the number of launches (2).
 int  launch_residual(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b,
                      const float *p_r, const float *p_b, double *partials, int max_partials,
-                     double *out2, cudaStream_t st);
+                     double *out2, cudaStream_t st, const LoopCheck *loop = nullptr);
 int  residual_blocks(const Geom &g);
 // z-slab decomposition of a solve.  slab_pass_supported: the temporal-blocking
 // pass applies to g.  launch_tb_pass_slab: one pass (two sweeps) over planes
@@ -146,14 +162,15 @@ void launch_gradient(const Geom &g, const SolveParams &sp, float dt_over_rho_dx,
 // remainder.
 int  launch_defect(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, const float *p_r,
                    const float *p_b, const float *d_r, const float *d_b, float *def_r, float *def_b, double *partials,
-                   int max_partials, double *out2, cudaStream_t st);
+                   int max_partials, double *out2, cudaStream_t st, const LoopCheck *loop = nullptr);
 // The arrays of a defect-correction solve (build_solve_graph): its checks
 // fold d into p and form a fresh defect instead of a plain residual.
 struct DefectArrays {
     const float *rhs_r, *rhs_b;
     float *p_r, *p_b, *d_r, *d_b, *df_r, *df_b;
 };
-void launch_fold(const Geom &g, float *p_r, float *p_b, float *d_r, float *d_b, cudaStream_t st);
+void launch_fold(const Geom &g, float *p_r, float *p_b, float *d_r, float *d_b, cudaStream_t st,
+                 const LoopCheck *loop = nullptr);
 // Packed <-> natural layout.
 void launch_pack(const Geom &g, const float *nat, float *red, float *black, cudaStream_t st);
 void launch_unpack(const Geom &g, const float *red, const float *black, float *nat,
@@ -161,13 +178,6 @@ void launch_unpack(const Geom &g, const float *red, const float *black, float *n
 
 void launch_perlin(const float *pos3, int n, float scale, int seed, float *out, cudaStream_t st);
 
-// Device-side state of a graph-run solve (see graph_solve.cu).
-struct SolveCtl {
-    int iters, checks, converged, pad;
-    double r2, b2;                      // last ||r||^2, ||b||^2
-    unsigned long long sweep_ns, t0;    // global-timer time inside sweep batches
-    unsigned long long check_ns, t1;    // ... and inside the residual checks
-};
 cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b,
                               float *p_r, float *p_b, double *partials, int n_partials, double *norm2,
                               SolveCtl *ctl, int chunk, int max_iter, double tol, int variant, cudaStream_t st,
