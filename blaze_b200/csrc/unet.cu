@@ -64,8 +64,9 @@ size_t tensor_voxels(const LDims &d) {
 struct CellArr {
     const float *r, *b;
     __device__ __forceinline__ float at(int i, int j, int k, int W, int H) const {
-        if (!b) return __ldg(r + lin(i, j, k, W, H));
-        return __ldg((((i + j + k) & 1) ? b : r) + pidx(i, j, k, W >> 1, H));
+        const unsigned row = (unsigned)(j + H * k);         // 32-bit indices, as split3's
+        if (!b) return __ldg(r + ((unsigned)i + (unsigned)W * row));
+        return __ldg((((i + j + k) & 1) ? b : r) + ((unsigned)(i >> 1) + (unsigned)(W >> 1) * row));
     }
 };
 

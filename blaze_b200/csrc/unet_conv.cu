@@ -68,9 +68,10 @@ __device__ __forceinline__ unsigned long long conv_now_ns() {
 constexpr unsigned long long kConvWaitNs = 10ull * 1000ull * 1000ull;
 
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int *err) {
-    // Bounded in time (device global timer): gives up after kConvWaitNs,
-    // records the timeout and returns.
-    const unsigned long long t0 = conv_now_ns();
+    // Bounded in time (device global timer, read only when the first tries
+    // fail: the read is slow): gives up after kConvWaitNs, records the timeout
+    // and returns.
+    unsigned long long t0 = 0;
     for (;;) {
         for (int it = 0; it < 64; ++it) {
             uint32_t done;
@@ -79,7 +80,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, int *e
                          : "=r"(done) : "r"(mbar), "r"(parity) : "memory");
             if (done) return true;
         }
-        if (conv_now_ns() - t0 > kConvWaitNs) break;
+        const unsigned long long t = conv_now_ns();
+        if (t0 == 0) t0 = t;
+        else if (t - t0 > kConvWaitNs) break;
     }
     if (err) atomicExch(err, 1);
     return false;
@@ -232,65 +235,81 @@ k_conv3d_tc(int W, int H, int D, int cin, int out_stride, int out_offset, const 
 int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 
 // ---------------------------------------------------------------------------
-// z-marching variant for layers with cin, cout in {16, 32} (the full- and
-// half-resolution layers, which carry most of the network's voxels).  A CTA
-// keeps the layer's weights resident in shared memory and walks one 128-voxel
-// tile through `zs` consecutive planes.  Output plane z needs input planes
-// z-1, z, z+1 (padded planes z, z+1, z+2), 3 rows each.  They arrive by TMA
-// (one tensor-map box per row, completing on the slot's mbarrier by
-// transaction count) in a ring of S plane slots, S - 2 planes ahead, so each
-// plane's rows are staged once per tile and their latency is hidden behind
-// several planes; the TMEM accumulator has kZmAcc buffers.  The CTA is warp
-// specialised and its warps hand over through mbarriers only:
-//   workers (warps 0-3), iteration z: thread 0 issues the copies of padded
-//   plane z+S-2 (into the slot of plane z-2, whose last reader, plane z-2's
-//   MMAs, completed before the workers read that plane out) | all wait for
-//   plane z-1's MMAs (accf), read its accumulator from TMEM, add bias /
-//   ReLU, store, arrive on acce (buffer free);
-//   MMA warp (warp 4), iteration z: wait full[] of plane z+2 and acce of
-//   buffer z % kZmAcc (read out by iteration z-kZmAcc) | lane 0 issues
-//   27 x cin/16 MMAs into that buffer and commits to its accf.
-// So the MMA warp runs up to kZmAcc - 1 planes ahead of the workers.  Every
-// wait is bounded in time; a wait that gives up sets the error flag and ends
-// that warp's loop, which ends the others' at their next (bounded) wait;
-// before the CTA ends, the MMA warp waits for its last commit and thread 0
-// for the latest copy into every slot.
-// S is as many slots as fit, at most 8: with two CTAs per SM when at least 6
-// fit in half the SM's shared memory (two independent pipelines), else with
-// one CTA.
+// z-marching variant for the layers with 16 to 64 input and output channels
+// whose weights fit in shared memory (they carry nearly all of the network's
+// voxels).  A CTA keeps the layer's weights resident and walks a tile of 8 x 16
+// voxels (x, y) through `zs` output planes.
+//
+// What bounds such a layer is the number of MMAs: with 16 output channels one
+// of 128 x 16 x 16 takes as long as one three times as wide, since both read the
+// same 128 x 16 operand of voxels.  So each staged block, the 16-channel chunk c
+// of input plane p, is used once, for the three output planes it reaches: an
+// MMA per (dy, dx) with N = 3 Cout, the weights of dz = +1, 0, -1 side by side
+// and the accumulators of output planes p - 1, p, p + 1 side by side in a TMEM
+// ring of R planes.  9 MMAs instead of 27 (10, since a new plane's first one
+// overwrites while the others add).  Chunk c runs 2 c planes behind chunk 0, so
+// every output still adds its taps in the general kernel's order, chunk by chunk
+// and tap by tap, and has its bits.
+//
+// A tile of 8 x 16 voxels instead of 128 in a row reads 1.4 input voxels per
+// output voxel and plane, not 3, and its block arrives by TMA as one box of 10 x
+// 18 voxels in the canonical K-major layout (core matrices of 8 voxels, 160 bytes
+// from row to row): tap (dy, dx) is the same block seen 160 dy + 16 dx bytes on.
+//
+// Warps: four read finished accumulators out of TMEM, add bias / ReLU and store;
+// one issues the MMAs (the whole warp runs the loop, so descriptors are uniform
+// values, and one elected lane's instructions take effect); one issues the
+// copies.  They hand over through mbarriers only: full / empty per ring slot,
+// done / free per accumulator.  Every wait is bounded in time; a wait that gives
+// up sets the error flag and ends that warp's loop, which ends the others' at
+// their next wait; before the CTA ends, the MMA warp waits for its last commit
+// and the copy warp for every copy it issued.
+//
+// Measured (16 -> 16 at 256^3, 32 -> 16 at 256^3, 32 -> 32 at 128^3, 64 -> 32 at
+// 128^3): 461, 786, 139 and 360 us; with an MMA per tap and output plane on 128
+// voxels of a row 738, 1994, 298 and (general kernel) 1146 us.  What bounds it
+// now: the copies, whose innermost run is 16 bytes (344 us of the 461 remain
+// without the MMAs and the epilogue), then the MMAs.
 // ---------------------------------------------------------------------------
-constexpr int kZmWorkers = 128;                           // staging + epilogue warps 0-3
-constexpr int kZmThreads = kZmWorkers + 32;               // + the MMA warp
-constexpr int kZmAcc = 4;                                 // accumulator buffers in TMEM
-constexpr int kZmSmemOne = 227 * 1024 - 1024;            // dynamic bytes, one CTA per SM
-constexpr int kZmSmemTwo = 228 * 1024 / 2 - 1024 - 128;  // dynamic bytes, two CTAs per SM
+constexpr int kZmWorkers = 128;                           // epilogue warps 0-3
+constexpr int kZmThreads = kZmWorkers + 64;               // + the MMA warp + the copy warp
+constexpr int kZmTX = 8, kZmTY = 16;                      // tile (x, y)
+constexpr int kZmRow = (kZmTX + 2) * 16;                  // bytes of one row of a block's half
+constexpr int kZmHalf = (kZmTY + 2) * kZmRow;             // 8 channels of a block
+constexpr int kZmBlock = 2 * kZmHalf;                     // 16 channels of 10 x 18 voxels
+constexpr int kZmSmemOne = 227 * 1024 - 1024;             // dynamic bytes, one CTA per SM
+constexpr int kZmSmemTwo = 228 * 1024 / 2 - 1024 - 512;   // dynamic bytes, two CTAs per SM
+constexpr int kZmMaxSlots = 12;
+static_assert(kZmBlock % 128 == 0, "128-byte aligned ring slots");
 
-// A slot holds the rows dy = -1, 0, 1 of one padded plane, each row block
-// [ch][kg][v][8 channels] (CIN/16 chunks of two 8-channel halves of 130
-// voxels) as one TMA box, the blocks 128-byte aligned.
-template <int CIN> __host__ __device__ constexpr int zm_dy_bytes() { return ((CIN / 16) * kRowBytes + 127) & ~127; }
-template <int CIN> __host__ __device__ constexpr int zm_slot_bytes() { return 3 * zm_dy_bytes<CIN>(); }
-template <int N, int CIN> __host__ __device__ constexpr int zm_w_bytes() { return 27 * (CIN / 16) * N * 32; }
-// dynamic shared memory besides the slots: the weights and 128 bytes of
-// alignment slack
-template <int N, int CIN> __host__ __device__ constexpr int zm_fixed_bytes() { return zm_w_bytes<N, CIN>() + 128; }
-template <int N, int CIN> __host__ __device__ constexpr int zm_slots() {
-    return (kZmSmemTwo - zm_fixed_bytes<N, CIN>()) / zm_slot_bytes<CIN>() >= 6
-               ? ((kZmSmemTwo - zm_fixed_bytes<N, CIN>()) / zm_slot_bytes<CIN>() > 8
-                      ? 8 : (kZmSmemTwo - zm_fixed_bytes<N, CIN>()) / zm_slot_bytes<CIN>())
-               : ((kZmSmemOne - zm_fixed_bytes<N, CIN>()) / zm_slot_bytes<CIN>() > 8
-                      ? 8 : (kZmSmemOne - zm_fixed_bytes<N, CIN>()) / zm_slot_bytes<CIN>());
+template <int N, int CIN> struct Zm {
+    static constexpr int CH = CIN / 16;
+    static constexpr int kWeights = 27 * CH * N * 32;
+    // output planes in flight: 3 for a plane's own MMAs, 2 per later chunk, and
+    // at least 3 being read out; a power of two
+    static constexpr int R = 2 * (CH - 1) + 6 <= 8 ? 8 : 16;
+    static constexpr int kCols = R * N;
+    static constexpr bool kTwo = kCols <= 256 && kWeights + 128 + 6 * kZmBlock <= kZmSmemTwo;   // CTAs per SM
+    static constexpr int kRoom = ((kTwo ? kZmSmemTwo : kZmSmemOne) - kWeights - 128) / kZmBlock;
+    static constexpr int SL = kRoom < kZmMaxSlots ? kRoom : kZmMaxSlots;
+    static constexpr int kSmem = kWeights + 128 + SL * kZmBlock;
+    static_assert(kCols <= 512 && SL >= 4, "TMEM columns and ring slots");
+};
+
+// One tcgen05.mma, by the lane whose `lead` is set; descriptors as 32-bit halves
+// (offsets only move the address field, in the low half).
+__device__ __forceinline__ void zm_mma(uint32_t lead, uint32_t d, uint32_t a, uint32_t a_hi, uint32_t b, uint32_t b_hi,
+                                       uint32_t idesc, uint32_t acc) {
+    asm volatile("{\n .reg .pred p, q;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n setp.ne.b32 q, %7, 0;\n"
+                 " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
+                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(a_hi), "r"(b), "r"(b_hi), "r"(idesc), "r"(acc), "r"(lead) : "memory");
 }
-template <int N, int CIN> __host__ __device__ constexpr int zm_smem_bytes() {
-    return zm_fixed_bytes<N, CIN>() + zm_slots<N, CIN>() * zm_slot_bytes<CIN>();
+__device__ __forceinline__ void zm_commit(uint32_t lead, uint32_t bar) {
+    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
+                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
+                 ::"r"(bar), "r"(lead) : "memory");
 }
-static_assert(zm_w_bytes<16, 16>() % 128 == 0 && zm_w_bytes<32, 32>() % 128 == 0 && zm_dy_bytes<16>() == 4224 &&
-                  zm_dy_bytes<32>() == 8320, "128-byte aligned slots");
-static_assert(zm_slots<16, 16>() == 8 && zm_slots<32, 16>() == 6 && zm_slots<16, 32>() == 8 &&
-                  zm_slots<32, 32>() == 7, "ring slots of the z-marching convolution");
-static_assert(zm_smem_bytes<16, 16>() <= kZmSmemTwo && zm_smem_bytes<32, 16>() <= kZmSmemTwo &&
-                  zm_smem_bytes<16, 32>() <= kZmSmemOne && zm_smem_bytes<32, 32>() <= kZmSmemOne,
-              "shared memory of the z-marching convolution");
 
 template <int N, int CIN, bool RELU>
 __global__ void __launch_bounds__(kZmThreads, 1)
@@ -298,116 +317,84 @@ k_conv3d_zm(int W, int H, int D, int zs, int out_stride, int out_offset, const _
             const __nv_bfloat16 *__restrict__ w, const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y,
             const __nv_bfloat16 *__restrict__ aux, int *err) {
     extern __shared__ __align__(128) unsigned char smem[];
-    constexpr int CH = CIN / 16;
-    constexpr int S = zm_slots<N, CIN>();
-    constexpr int kSlot = zm_slot_bytes<CIN>();
-    constexpr int kDy = zm_dy_bytes<CIN>();
-    constexpr uint32_t kSlotTx = 3u * CH * kRowBytes;       // bytes the three row boxes of a plane bring
-    constexpr int kCols = kZmAcc * N < 32 ? 32 : kZmAcc * N;   // a power of two
-    constexpr uint32_t idesc = umma_idesc_bf16(kConvM, N);
-    // full[s]: the plane in ring slot s has landed (the TMA copies' bytes);
-    // accf[b]: the MMAs into accumulator buffer b completed (their commit);
-    // acce[b]: buffer b has been read out (one arrival per worker).  Plane
-    // iteration it uses buffer it % kZmAcc, the n-th time for n = it / kZmAcc.
-    __shared__ __align__(8) uint64_t full[S], accf[kZmAcc], acce[kZmAcc];
+    typedef Zm<N, CIN> Z;
+    constexpr int CH = Z::CH, R = Z::R, SL = Z::SL;
+    constexpr int kTap = 3 * N * 32;                      // bytes of one (chunk, dy, dx)'s weights
+    __shared__ __align__(8) uint64_t full[SL], empty[SL], accf[R], acce[R], fin;
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool worker = warp < 4;
     const int Wp = W + 2, Hp = H + 2;
-    const long long plane = (long long)Wp * Hp;
-    const long long P0 = (long long)Wp + (long long)kConvM * blockIdx.x;
-    const int z0 = blockIdx.y * zs;
+    const int X0 = blockIdx.x * kZmTX, Y0 = blockIdx.y * kZmTY, z0 = blockIdx.z * zs;
     const int nz = (z0 + zs < D ? z0 + zs : D) - z0;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                     ::"r"(smem_u32(&tmem_base)), "r"(kCols) : "memory");
+                     ::"r"(smem_u32(&tmem_base)), "r"(Z::kCols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int s = 0; s < S; ++s)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&full[s])) : "memory");
-        for (int b = 0; b < kZmAcc; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&accf[b])) : "memory");
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&acce[b])), "r"(kZmWorkers) : "memory");
-        }
+        auto init = [](uint64_t *b, int n) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n) : "memory");
+        };
+        for (int s = 0; s < SL; ++s) { init(&full[s], 1); init(&empty[s], 1); }
+        for (int b = 0; b < R; ++b) { init(&accf[b], 1); init(&acce[b], kZmWorkers); }
+        init(&fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    const uint32_t bS = (smem_u32(smem) + 127u) & ~127u;  // weights, then the ring, 128-byte aligned
+    const uint32_t aS = bS + (uint32_t)Z::kWeights;
+    // Weights: per (chunk, dy, dx) 3 N rows of 16 channels, K-major: the rows of
+    // output plane p - 1 (dz = +1), p (0), p + 1 (-1).
+    for (int e = tid; e < 27 * CH * N * 2; e += kZmThreads) {
+        const int kg = e & 1, n = (e >> 1) % N, ct = (e >> 1) / N;          // ct = ch * 27 + tap
+        const int ch = ct / 27, t = ct % 27, o = 2 - t / 9, t9 = t % 9;
+        cp_async16(bS + (ch * 9 + t9) * kTap + kg * 3 * N * 16 + (o * N + n) * 16,
+                   w + ((size_t)t * N + n) * CIN + ch * 16 + kg * 8);
+    }
+    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base;
-    const uint32_t bS = (smem_u32(smem) + 127u) & ~127u;       // weights, then the ring, 128-byte aligned
-    const uint32_t aS = bS + (uint32_t)zm_w_bytes<N, CIN>();
-    // Ring slot of padded plane pz: (pz - z0) % S, so the n-th fill of a slot
-    // is the plane z0 + s + n S and completes phase n of full[s].
-    auto slot_of = [&](int pz) { return (pz - z0) % S; };
-    auto fill_parity = [&](int pz) { return (uint32_t)(((pz - z0) / S) & 1); };
-    // Weights of every 16-channel chunk: block (ch, tap) = N rows x 32 B,
-    // K-major (cp.async by the workers, fenced to the async proxy before the
-    // barrier that starts the pipeline).
-    if (worker) {
-        for (int e = tid; e < 27 * CH * N * 2; e += kZmWorkers) {
-            const int kg = e & 1, n = (e >> 1) % N, ct = (e >> 1) / N;      // ct = ch * 27 + tap
-            const int ch = ct / 27, t = ct % 27;
-            cp_async16(bS + ct * N * 32 + kg * N * 16 + n * 16, w + ((size_t)t * N + n) * CIN + ch * 16 + kg * 8);
-        }
-        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    __syncthreads();
-    // Padded plane pz by TMA: rows dy = -1, 0, 1 of the tile (130 voxels
-    // each: its 128 and one either side, flattened in-plane index P0 - 1 +
-    // (dy - 1) Wp on), one box per row of 8 channels x 130 voxels x 2
-    // halves x 1 plane x CIN/16 chunks, landing as [ch][kg][v][8] at
-    // dy * kDy in the slot; voxels outside the plane read as zeros.
-    auto tma_plane = [&](int pz) {
-        const uint32_t bar = smem_u32(&full[slot_of(pz)]);
-        const uint32_t dst = aS + (uint32_t)(slot_of(pz) * kSlot);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kSlotTx) : "memory");
-#pragma unroll
-        for (int dy = 0; dy < 3; ++dy)
-            asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                         " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                         ::"r"(dst + (uint32_t)(dy * kDy)), "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(0),
-                           "r"((int)(P0 - 1) + (dy - 1) * Wp), "r"(0), "r"(pz), "r"(0), "r"(bar)
-                         : "memory");
-    };
-    int last_plane = z0 - 1;                             // last plane thread 0 asked for
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_base, 0);
+    // Blocks in order: round s takes chunk c of input plane z0 - 1 + s - 2 c, for
+    // the planes z0 - 1 .. z0 + nz.
+    const int rounds = nz + 2 + 2 * (CH - 1);
+    auto in_range = [&](int p) { return p >= z0 - 1 && p <= z0 + nz; };
 
-    if (worker) {
-        // ---- workers: thread 0 issues the plane copies; all drain the
-        // accumulators ----
-        // This thread's voxel of the tile (TMEM lane 32 * warp + lane) and
-        // the bias, the same on every plane.
-        const long long Pv = P0 + 32 * warp + lane;
-        const int yv = (int)(Pv / Wp), xv = (int)(Pv - (long long)yv * Wp);
-        const bool inside = xv >= 1 && xv <= W && yv >= 1 && yv <= H;
-        float bv[N];
-#pragma unroll
-        for (int q = 0; q < N; ++q) bv[q] = bias ? __ldg(bias + q) : 0.0f;
-        // Reads accumulator buffer it % kZmAcc (output plane z0 + it) and stores
-        // it; false (the whole warp alike) when its wait gave up.
-        auto epilogue = [&](int it) -> bool {
-            const bool done = mbar_wait(smem_u32(&accf[it % kZmAcc]), (uint32_t)((it / kZmAcc) & 1), err);
-            if (!__all_sync(0xffffffffu, done)) return false;
+    if (warp < 4) {
+        // ---- epilogue: this thread's voxel of the tile is TMEM lane tid ----
+        const int xv = X0 + (tid & 7), yv = Y0 + (tid >> 3);
+        const bool inside = xv < W && yv < H;
+        const long long plane = (long long)Wp * Hp, Pv = (long long)(yv + 1) * Wp + xv + 1;
+        bool ok = true;
+#pragma unroll 1
+        for (int it = 0; it < nz && ok; ++it) {
+            const int slot = it & (R - 1);
+            ok = __all_sync(0xffffffffu, mbar_wait(smem_u32(&accf[slot]), (uint32_t)((it / R) & 1), err));
+            if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const long long outv = (long long)(z0 + it + 1) * plane + Pv;
 #pragma unroll
             for (int n0 = 0; n0 < N; n0 += 16) {
                 uint32_t r[16];
-                const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)((it % kZmAcc) * N + n0);
+                const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(slot * N + n0);
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
                              : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
                                "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
                                "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
                              : "r"(taddr) : "memory");
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (n0 + 16 == N) {
+                    // read out: the buffer may be overwritten
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acce[slot])) : "memory");
+                }
                 if (inside) {
                     float v[16];
 #pragma unroll
                     for (int q = 0; q < 16; ++q) {
-                        v[q] = __uint_as_float(r[q]) + bv[n0 + q];
+                        v[q] = __uint_as_float(r[q]) + (bias ? __ldg(bias + n0 + q) : 0.0f);
                         if (RELU) v[q] = fmaxf(v[q], 0.0f);
                     }
                     const long long o = outv * out_stride + out_offset + n0;
@@ -430,142 +417,168 @@ k_conv3d_zm(int W, int H, int D, int zs, int out_stride, int out_offset, const _
                     dst[1] = *reinterpret_cast<uint4 *>(&h[4]);
                 }
             }
-            // the buffer may be overwritten by the MMAs of iteration it + kZmAcc
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&acce[it % kZmAcc])) : "memory");
-            return true;
-        };
-        // Prologue: padded planes z0 .. z0+S-3 (those the tile needs).
-        if (tid == 0)
-            for (int p = 0; p < S - 2 && p < nz + 2; ++p) {
-                tma_plane(z0 + p);
-                last_plane = z0 + p;
-            }
-        bool ok = true;
-#pragma unroll 1
-        for (int it = 0; it < nz && ok; ++it) {
-            const int z = z0 + it;
-            // plane z+S-2 goes into the slot of plane z-2, whose last reader
-            // (the MMAs of iteration it-2) completed before this thread's
-            // epilogue(it-2) returned
-            if (tid == 0 && it + S - 2 < nz + 2) {
-                tma_plane(z + S - 2);
-                last_plane = z + S - 2;
-            }
-            if (it > 0) ok = epilogue(it - 1);
         }
-        if (ok && nz > 0) ok = epilogue(nz - 1);
-        if (!ok && err) atomicExch(err, 1);
-        // No copy may land after the CTA ends: thread 0 waits (bounded) for
-        // the latest fill of every slot it issued (done already unless a
-        // wait gave up).
-        if (tid == 0)
-            for (int p = last_plane; p >= z0 && p > last_plane - S; --p)
-                mbar_wait(smem_u32(&full[slot_of(p)]), fill_parity(p), nullptr);
-    } else {
-        // ---- MMA warp: lane 0 issues each plane's 27 x cin/16 MMAs ----
-        // Operand descriptors at the start of the plane ring and of the
-        // weights.  Every operand address stays below 2^18 bytes, so adding an
-        // offset's 16-byte units to the 14-bit address field never carries.
-        const uint64_t a_desc0 = umma_desc(aS, kKgBytes, 128);
-        const uint64_t b_desc0 = umma_desc(bS, N * 16, 128);
-        int issued = 0;
+    } else if (warp == 4) {
+        // ---- MMA warp ----
+        // Every operand address stays below 2^18 bytes, so adding an offset's
+        // 16-byte units to the 14-bit address field never carries.
+        const uint64_t a_desc0 = umma_desc(aS, kZmHalf, kZmRow), b_desc0 = umma_desc(bS, 3 * N * 16, 128);
+        const uint32_t a_lo = (uint32_t)a_desc0, a_hi = (uint32_t)(a_desc0 >> 32);
+        const uint32_t b_lo = (uint32_t)b_desc0, b_hi = (uint32_t)(b_desc0 >> 32);
+        const uint32_t lead = lane == 0 ? 1u : 0u;
         bool ok = true;
+        int n = 0, slot = 0;                              // blocks taken; the next one's ring slot
+        uint32_t phase = 0;
 #pragma unroll 1
-        for (int it = 0; it < nz && ok; ++it) {
-            const int z = z0 + it;
-            bool done = true;
-            if (it == 0) {
-                done = mbar_wait(smem_u32(&full[slot_of(z)]), fill_parity(z), err) && done;
-                done = mbar_wait(smem_u32(&full[slot_of(z + 1)]), fill_parity(z + 1), err) && done;
-            }
-            done = mbar_wait(smem_u32(&full[slot_of(z + 2)]), fill_parity(z + 2), err) && done;
-            // accumulator buffer it % kZmAcc was last read out by epilogue(it - kZmAcc)
-            if (it >= kZmAcc)
-                done = mbar_wait(smem_u32(&acce[it % kZmAcc]), (uint32_t)(((it - kZmAcc) / kZmAcc) & 1), err) && done;
-            if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
-                const uint32_t acc = tmem + (uint32_t)((it % kZmAcc) * N);
-                // descriptors of the slots of padded planes z, z+1, z+2 (taps
-                // dz = -1, 0, +1); a tap's operand is its slot's descriptor
-                // plus a constant offset in the 16-byte address field
-                const uint64_t sz[3] = {a_desc0 + (uint64_t)((slot_of(z) * kSlot) >> 4),
-                                        a_desc0 + (uint64_t)((slot_of(z + 1) * kSlot) >> 4),
-                                        a_desc0 + (uint64_t)((slot_of(z + 2) * kSlot) >> 4)};
+        for (int s = 0; s < rounds && ok; ++s)
+#pragma unroll 1
+            for (int c = 0; c < CH; ++c) {
+                const int p = z0 - 1 + s - 2 * c;
+                if (!in_range(p)) continue;
+                bool done = mbar_wait(smem_u32(&full[slot]), phase, err);
+                // output planes lo .. hi as iterations of this CTA; the last is
+                // new where chunk 0 meets it for the first time
+                const int lo = p - 1 < z0 ? 0 : p - 1 - z0, hi = p + 1 > z0 + nz - 1 ? nz - 1 : p + 1 - z0;
+                const bool fresh = c == 0 && hi == p + 1 - z0;
+                if (fresh && hi >= R)
+                    done = mbar_wait(smem_u32(&acce[hi & (R - 1)]), (uint32_t)((hi / R - 1) & 1), err) && done;
+                if (!__all_sync(0xffffffffu, done)) { ok = false; break; }
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t ad0 = a_lo + (uint32_t)((slot * kZmBlock) >> 4);
+                // weights' rows start at output plane p - 1
+                const uint32_t bd0 = b_lo + (uint32_t)((c * 9 * kTap + (lo + z0 - (p - 1)) * N * 16) >> 4);
+                // the ring's end may split the columns of lo .. hi: `head` planes
+                // up to it, the rest from its start
+                const int first = lo & (R - 1), count = hi - lo + 1, head = first + count > R ? R - first : count;
+                const uint32_t d0 = tmem + (uint32_t)(first * N);
+                auto idesc = [&](int planes) { return umma_idesc_bf16(kConvM, 0) + ((uint32_t)(planes * N / 8) << 17); };
+                auto offset = [&](int planes) { return (uint32_t)(planes * N); };        // weights' rows, 16 bytes each
+                auto tap = [&](int t) { return (uint32_t)(((t / 3) * kZmRow + (t % 3) * 16) >> 4); };
+                int t0 = 0;
+                if (fresh) {                             // tap 0: the new plane overwrites, the others add
+                    const int old = count - 1, h = head < old ? head : old;
+                    if (h > 0) zm_mma(lead, d0, ad0, a_hi, bd0, b_hi, idesc(h), 1u);
+                    if (old > h) zm_mma(lead, tmem, ad0, a_hi, bd0 + offset(h), b_hi, idesc(old - h), 1u);
+                    zm_mma(lead, tmem + (uint32_t)((hi & (R - 1)) * N), ad0, a_hi, bd0 + offset(old), b_hi, idesc(1), 0u);
+                    t0 = 1;
+                }
+                const uint32_t id0 = idesc(head), id1 = idesc(count - head), bd1 = bd0 + offset(head);
+                if (head == count) {
+                    if (t0 == 0) zm_mma(lead, d0, ad0, a_hi, bd0, b_hi, id0, 1u);
 #pragma unroll
-                for (int ch = 0; ch < CH; ++ch) {
-#pragma unroll
-                    for (int t = 0; t < 27; ++t) {
-                        const int dzi = t / 9, dyi = (t / 3) % 3, dxi = t % 3;
-                        const uint64_t ad = sz[dzi] + (uint64_t)((dyi * kDy + ch * kRowBytes + dxi * 16) >> 4);
-                        const uint64_t bd = b_desc0 + (uint64_t)(((ch * 27 + t) * N * 32) >> 4);
-                        const uint32_t accum = (ch > 0 || t > 0) ? 1u : 0u;
-                        asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                                     " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                                     ::"r"(acc), "l"(ad), "l"(bd), "r"(idesc), "r"(accum) : "memory");
+                    for (int t = 1; t < 9; ++t)
+                        zm_mma(lead, d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
+                } else {
+#pragma unroll 1
+                    for (int t = t0; t < 9; ++t) {
+                        zm_mma(lead, d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
+                        zm_mma(lead, tmem, ad0 + tap(t), a_hi, bd1 + (uint32_t)((t * kTap) >> 4), b_hi, id1, 1u);
                     }
                 }
-                asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                             ::"r"(smem_u32(&accf[it % kZmAcc])) : "memory");
+                zm_commit(lead, smem_u32(&empty[slot]));
+                if (c == CH - 1 && p - 1 >= z0) zm_commit(lead, smem_u32(&accf[(p - 1 - z0) & (R - 1)]));
+                ++n;
+                if (++slot == SL) { slot = 0; phase ^= 1u; }
             }
-            __syncwarp();
-            issued = it + 1;
+        // The last MMAs complete before the accumulator columns are released,
+        // also when a wait gave up (bounded wait).
+        if (n > 0) {
+            zm_commit(lead, smem_u32(&fin));
+            mbar_wait(smem_u32(&fin), 0, nullptr);
         }
-        // The last committed MMAs complete before the accumulator columns are
-        // released, also when a worker's wait gave up (bounded wait).
-        if (issued > 0)
-            mbar_wait(smem_u32(&accf[(issued - 1) % kZmAcc]), (uint32_t)(((issued - 1) / kZmAcc) & 1), nullptr);
-        (void)ok;
+    } else if (lane == 0) {
+        // ---- copy warp ----
+        int n = 0, slot = 0;
+        uint32_t phase = 1;                               // a fresh barrier's previous phase has completed
+        bool ok = true;
+        for (int s = 0; s < rounds && ok; ++s)
+            for (int c = 0; c < CH; ++c) {
+                const int p = z0 - 1 + s - 2 * c;
+                if (!in_range(p)) continue;
+                if (!mbar_wait(smem_u32(&empty[slot]), phase, err)) { ok = false; break; }
+                const uint32_t bar = smem_u32(&full[slot]);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kZmBlock) : "memory");
+                asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                             " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
+                             ::"r"(aS + (uint32_t)(slot * kZmBlock)), "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(0),
+                               "r"(X0), "r"(Y0), "r"(2 * c), "r"(p + 1), "r"(bar)
+                             : "memory");
+                ++n;
+                if (++slot == SL) { slot = 0; phase ^= 1u; }
+            }
+        // No copy may land after the CTA ends (done already unless a wait gave up).
+        for (int q = n - 1; q >= 0 && q >= n - SL; --q)
+            mbar_wait(smem_u32(&full[q % SL]), (uint32_t)((q / SL) & 1), nullptr);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(Z::kCols) : "memory");
 }
 
-constexpr int kZmPlanes = 16;
-
 // Tensor map of a padded channels-last activation x (CIN channels, W+2 x
-// H+2 x D+2 voxels from x) for the z-marching convolution's row boxes:
-// dims (8 channels, in-plane voxel, 8-channel half, plane, 16-channel chunk)
-// with byte strides (2 CIN, 16, plane, 32), box (8, 130, 2, 1, CIN/16).  The
-// innermost coordinate of every copy is 0, so every copy starts 16-byte
-// aligned.
+// H+2 x D+2 voxels from x): dims (8 channels, x, y, 8-channel group, z) with
+// byte strides (2 CIN, row, 16, plane), box (8, 10, 18, 2, 1): one 16-channel
+// chunk of a tile with its border.  The innermost coordinate of every copy is
+// 0, so every copy starts 16-byte aligned; voxels past the tensor read as zeros.
 static bool zm_tensor_map(CUtensorMap *m, const __nv_bfloat16 *x, const ConvDesc &cd) {
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
     const cuuint64_t Wp = (cuuint64_t)cd.W + 2, Hp = (cuuint64_t)cd.H + 2, Dp = (cuuint64_t)cd.D + 2;
     const cuuint64_t C = (cuuint64_t)cd.cin;
-    const cuuint64_t dims[5] = {8, Wp * Hp, 2, Dp, C / 16};
-    const cuuint64_t strides[4] = {C * 2, 16, Wp * Hp * C * 2, 32};
-    const cuuint32_t box[5] = {8, (cuuint32_t)kRowVox, 2, 1, (cuuint32_t)(C / 16)};
+    const cuuint64_t dims[5] = {8, Wp, Hp, C / 8, Dp};
+    const cuuint64_t strides[4] = {C * 2, Wp * C * 2, 16, Wp * Hp * C * 2};
+    const cuuint32_t box[5] = {8, kZmTX + 2, kZmTY + 2, 2, 1};
     const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(x), dims, strides, box, estr,
                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+static int conv_sm_count() {
+    static int cache[64] = {0};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) dev = 0;
+    if (cache[dev] == 0) {
+        int n = 0;
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        cache[dev] = n > 0 ? n : 148;
+    }
+    return cache[dev];
+}
+
 template <int N, int CIN, bool RELU>
 static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
                              void *y, const __nv_bfloat16 *aux, int *err, cudaStream_t st) {
-    constexpr int smem = zm_smem_bytes<N, CIN>();
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_zm<N, CIN, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    typedef Zm<N, CIN> Z;
+    cudaError_t e = cudaFuncSetAttribute(k_conv3d_zm<N, CIN, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z::kSmem);
     if (e != cudaSuccess) return e;
     CUtensorMap xm;
     if (!zm_tensor_map(&xm, x, cd)) return cudaErrorNotSupported;
-    const long long interior = (long long)(cd.W + 2) * cd.H;
-    const dim3 grid((unsigned)((interior + kConvM - 1) / kConvM), (unsigned)((cd.D + kZmPlanes - 1) / kZmPlanes));
+    // Output planes per CTA: the least time of a whole number of waves, a CTA of
+    // zs planes taking zs + 2 + 2 (CH - 1) rounds and about 6 more to start.
+    const long long tiles = (long long)((cd.W + kZmTX - 1) / kZmTX) * ((cd.H + kZmTY - 1) / kZmTY);
+    const long long room = (long long)conv_sm_count() * (Z::kTwo ? 2 : 1);
+    int zs = 0;
+    long long best = 0;
+    for (int v = 4; v <= 64; v <<= 1) {
+        const long long ctas = tiles * ((cd.D + v - 1) / v), cost = (ctas + room - 1) / room * (v + 2 * Z::CH + 6);
+        if (zs == 0 || cost < best) { zs = v; best = cost; }
+    }
+    const dim3 grid((unsigned)((cd.W + kZmTX - 1) / kZmTX), (unsigned)((cd.H + kZmTY - 1) / kZmTY),
+                    (unsigned)((cd.D + zs - 1) / zs));
     const int os = cd.out_stride > 0 ? cd.out_stride : cd.cout;
-    k_conv3d_zm<N, CIN, RELU><<<grid, kZmThreads, smem, st>>>(cd.W, cd.H, cd.D, kZmPlanes, os, cd.out_offset, xm, w, bias,
-                                                       static_cast<__nv_bfloat16 *>(y), aux, err);
+    k_conv3d_zm<N, CIN, RELU><<<grid, kZmThreads, Z::kSmem, st>>>(cd.W, cd.H, cd.D, zs, os, cd.out_offset, xm, w, bias,
+                                                                  static_cast<__nv_bfloat16 *>(y), aux, err);
     return cudaGetLastError();
 }
 
-// The z-marching kernel for cin, cout in {16, 32} and BF16 output.
+// The z-marching kernel: BF16 output and a pair of channel counts whose weights
+// and accumulators fit.
 static bool zm_dispatch(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
                         void *y, const __nv_bfloat16 *aux, int *err, cudaStream_t st, cudaError_t *res) {
-    if (cd.out_f32 || (cd.cin != 16 && cd.cin != 32) || (cd.cout != 16 && cd.cout != 32)) return false;
+    if (cd.out_f32) return false;
 #define BLZ_ZM(NN, CC)                                                                              \
     if (cd.cout == NN && cd.cin == CC) {                                                            \
         *res = cd.relu ? launch_zm<NN, CC, true>(cd, x, w, bias, y, aux, err, st)                   \
@@ -576,6 +589,8 @@ static bool zm_dispatch(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_b
     BLZ_ZM(16, 32)
     BLZ_ZM(32, 16)
     BLZ_ZM(32, 32)
+    BLZ_ZM(32, 64)
+    BLZ_ZM(64, 32)
 #undef BLZ_ZM
     return false;
 }
