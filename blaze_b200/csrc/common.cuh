@@ -60,45 +60,6 @@ __device__ __forceinline__ float trilinear(const FieldRef &f, float inv_dx, floa
          + fz * ((1.0f - fy) * (a001 * (1.0f - fx) + a101 * fx) + fy * (a011 * (1.0f - fx) + a111 * fx));
 }
 
-// Lagrange cubic on nodes -1, 0, 1, 2 (src/Grid.h:148-163).
-__device__ __forceinline__ float cerp(float q0, float q1, float q2, float q3, float s) {
-    const float s2 = s * s, s3 = s2 * s;
-    return (-1.0f / 3.0f * s + 0.5f * s2 - 1.0f / 6.0f * s3) * q0
-         + (1.0f - s2 + 0.5f * (s3 - s)) * q1
-         + (s + 0.5f * (s2 - s3)) * q2
-         + (1.0f / 6.0f * (s3 - s)) * q3;
-}
-
-// Separable tricubic (x, then y, then z) with edge-clamped stencil indices;
-// CLAMP zeroes negatives after every 1-D stage (src/Grid.h:165-222).
-template <bool CLAMP>
-__device__ __forceinline__ float tricubic(const FieldRef &f, float inv_dx, float px, float py, float pz) {
-    const float gX = clamp_coord(px * inv_dx - f.ox, f.w);
-    const float gY = clamp_coord(py * inv_dx - f.oy, f.h);
-    const float gZ = clamp_coord(pz * inv_dx - f.oz, f.d);
-    const int i1 = (int)gX, j1 = (int)gY, k1 = (int)gZ;
-    const int i0 = max(i1 - 1, 0), i2 = i1 + 1, i3 = min(i1 + 2, f.w - 1);
-    const float sx = gX - (float)i1, sy = gY - (float)j1, sz = gZ - (float)k1;
-    const int rs = f.w, ps = f.w * f.h;             // 32-bit offsets, as in trilinear
-    float zs[4];
-#pragma unroll
-    for (int kk = 0; kk < 4; ++kk) {
-        const int kz = kk == 0 ? max(k1 - 1, 0) : kk == 3 ? min(k1 + 2, f.d - 1) : k1 + kk - 1;
-        float ys[4];
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-            const int jy = jj == 0 ? max(j1 - 1, 0) : jj == 3 ? min(j1 + 2, f.h - 1) : j1 + jj - 1;
-            const float *row = f.a + (rs * jy + ps * kz);
-            float v = cerp(ldg(row + i0), ldg(row + i1), ldg(row + i2), ldg(row + i3), sx);
-            ys[jj] = CLAMP ? fmaxf(v, 0.0f) : v;
-        }
-        const float v = cerp(ys[0], ys[1], ys[2], ys[3], sy);
-        zs[kk] = CLAMP ? fmaxf(v, 0.0f) : v;
-    }
-    const float v = cerp(zs[0], zs[1], zs[2], zs[3], sz);
-    return CLAMP ? fmaxf(v, 0.0f) : v;
-}
-
 __device__ __forceinline__ float len3(float x, float y, float z) { return sqrtf(x * x + y * y + z * z); }
 
 // ---------------------------------------------------------------------------
