@@ -653,11 +653,12 @@ static int choose_variant(blz_solver *s) {
     if (s->res.work) cand = {0, 4, kResidentVariant};
     else for (int v = 0; v < nv; ++v) cand.push_back(v);
     const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D * 2 + (nv > kSegVariants ? 1 : 0));
-    const std::string fkey = tune_key(s->device, s->g, nv, s->res.work != nullptr);
+    std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) { s->variant = it->second; return BLZ_OK; }
+        fkey = tune_key(s->device, s->g, nv, s->res.work != nullptr);
         const int v = tune_file_lookup(fkey);
         if ((v >= 0 && v < nv) || (v == kResidentVariant && s->res.work)) {
             g_tune_cache[key] = v;
