@@ -42,6 +42,11 @@
 // waiting for the rest of the launch and keeps sending, so the other CTAs do
 // not wait for it, and the solver reports BLZ_ERR_TIMEOUT.
 //
+// Widths that are not multiples of 8 (RAGGED): the last quad of a row is partly
+// pad, which the count 0 keeps at 0, and rows are read and written cell by cell,
+// once per batch of sweeps.  The counts per lane cost the update 10 to 20 %
+// (100^3 3.6 us a sweep, 96^3 2.75); one cell per thread takes 13.8 there.
+//
 // The operations per cell are gs_quad's, so the bits are those of the segment
 // kernel's sweeps.
 //
@@ -124,14 +129,58 @@ __device__ __forceinline__ Border res_border_row(int b, int TY, int TZ) {
     return {y, hi ? TZ + layer : -1 - layer, 0, hi ? 1 : -1, hi ? b - TY : b + TY};
 }
 
-template <int RZ, bool WARPROW>
+// One packed row quad from global memory.  RAGGED: rows of W / 2 cells that are
+// not whole quads (nor 16-byte aligned); the lanes past the row read 0.
+template <bool RAGGED>
+__device__ __forceinline__ float4 res_load(const float *p, int lanes) {
+    if (!RAGGED) return __ldcg(reinterpret_cast<const float4 *>(p));
+    float4 v = make_float4(__ldcg(p), 0.f, 0.f, 0.f);
+    if (lanes > 1) v.y = __ldcg(p + 1);
+    if (lanes > 2) v.z = __ldcg(p + 2);
+    if (lanes > 3) v.w = __ldcg(p + 3);
+    return v;
+}
+template <bool RAGGED>
+__device__ __forceinline__ void res_store(float *p, float4 v, int lanes) {
+    if (!RAGGED) { *reinterpret_cast<float4 *>(p) = v; return; }
+    p[0] = v.x;
+    if (lanes > 1) p[1] = v.y;
+    if (lanes > 2) p[2] = v.z;
+    if (lanes > 3) p[3] = v.w;
+}
+
+// gs_quad with a count per lane: `in` inside the row, `end` in the cell at the
+// row's end (lane 0 of its first quad where s = 0, the last valid lane of its
+// last where s = 1), 0 past it, so that the pad stays 0.
+__device__ __forceinline__ float4 res_quad_ragged(float scale, int s, float4 r, float4 o, float xe, float4 ym, float4 yp,
+                                                  float4 zm, float4 zp, float2 in, float2 end, bool first, bool last,
+                                                  int lanes) {
+    auto pick = [&](int t) {
+        const bool at_end = s == 0 ? first && t == 0 : last && t == lanes - 1;
+        return t >= lanes ? make_float2(0.0f, 0.0f) : at_end ? end : in;
+    };
+    const float2 d0 = pick(0), d1 = pick(1), d2 = pick(2), d3 = pick(3);
+    const f2_t sc = f2(scale, scale);
+    const f2_t xl01 = s == 0 ? f2(xe, o.x) : f2(o.x, o.y), xl23 = s == 0 ? f2(o.y, o.z) : f2(o.z, o.w);
+    const f2_t xr01 = s == 0 ? f2(o.x, o.y) : f2(o.y, o.z), xr23 = s == 0 ? f2(o.z, o.w) : f2(o.w, xe);
+    const f2_t a = gs_pair(sc, f2(r.x, r.y), xl01, xr01, f2(ym.x, ym.y), f2(yp.x, yp.y), f2(zm.x, zm.y),
+                           f2(zp.x, zp.y), f2(d0.x, d1.x), f2(d0.y, d1.y));
+    const f2_t b = gs_pair(sc, f2(r.z, r.w), xl23, xr23, f2(ym.z, ym.w), f2(yp.z, yp.w), f2(zm.z, zm.w),
+                           f2(zp.z, zp.w), f2(d2.x, d3.x), f2(d2.y, d3.y));
+    float4 out;
+    f2_split(a, out.x, out.y);
+    f2_split(b, out.z, out.w);
+    return out;
+}
+
+template <int RZ, bool WARPROW, bool RAGGED>
 __global__ void __launch_bounds__(res_threads<RZ>(), 1)
 k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
                 float *p_r, float *p_b, int sweeps, ResParams rs) {
     extern __shared__ __align__(16) float4 sm[];
     __shared__ float2 inv[8];
     constexpr int NR = RZ == 2 ? kResRecv2 : kResRecv4;
-    const int Wh = g.W >> 1, Wq = Wh >> 2, TY = rs.TY, TZ = rs.TZ, NRP = TY >> 1, nthr = blockDim.x;
+    const int Wh = g.W >> 1, Wq = (Wh + 3) >> 2, TY = rs.TY, TZ = rs.TZ, NRP = TY >> 1, nthr = blockDim.x;
     const int by = blockIdx.x % rs.NY, bz = blockIdx.x / rs.NY;
     const int mq = threadIdx.x % Wq, rp = (threadIdx.x / Wq) % NRP, zg = threadIdx.x / (Wq * NRP);
     const bool live = zg * RZ < TZ;                      // threads beyond the tile only exchange
@@ -139,6 +188,7 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
     const bool okA = live && jA < g.H, okB = live && jA + 1 < g.H;
     const int pl = Wh * g.H, gA = 4 * mq + Wh * jA + pl * k0;    // element offset of row A, plane k0
     const bool first = mq == 0, last = mq == Wq - 1;
+    const int tail = Wh - 4 * (Wq - 1), lanes = last ? tail : 4;     // valid cells of the last quad; of this thread's
     const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
     // Shared memory: p of both colours on planes -2..TZ+1 and rows -2..TY+1;
     // rhs of the tile; rhs of the red ring; the tables.
@@ -151,7 +201,7 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
     int *const t_dst = reinterpret_cast<int *>(ring_rhs + 2 * ring); // border quad: its place in the tile (-1: none)
     int *const t_src = t_dst + border, *const t_to = t_src + border; // what is sent for it and where to
     float4 *const ring_den = ring_rhs + ring;                        // reciprocals (hi, lo) inside the quad and at the row's end
-    int *const t_cell = t_to + border;                               // ring quad: parity, row ends
+    int *const t_cell = t_to + border;                               // ring quad: parity, at its row's end (x neighbour missing), last quad
 
     for (int q = threadIdx.x; q < 2 * pcol; q += nthr) sm[q] = zero4;
     if (threadIdx.x < 8)
@@ -180,13 +230,14 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
         // The border's first black values come from p itself: no CTA writes p
         // before every neighbour has sent its first sweep's.
         const long long e = 4 * m + (long long)Wh * j + (long long)pl * k;
-        if (in) sm[pcol + quad(b.y, b.z, m)] = __ldcg(reinterpret_cast<const float4 *>(p_b + e));
+        const int valid = m == Wq - 1 ? tail : 4;
+        if (in) sm[pcol + quad(b.y, b.z, m)] = res_load<RAGGED>(p_b + e, valid);
         if (q < ring) {
             const int s = (j + k) & 1, n = 2 + count_y(j) + count_z(k);
             const int end = n - (s ? (m == Wq - 1 ? x_hi : 0) : (m == 0 ? x_lo : 0));
-            t_cell[q] = in ? s | ((s ? m == Wq - 1 : m == 0) ? 2 : 0) : -1;
+            t_cell[q] = in ? s | ((s ? m == Wq - 1 : m == 0) ? 2 : 0) | (m == Wq - 1 ? 4 : 0) : -1;
             if (in) {
-                ring_rhs[q] = ld4(rhs_r + e);
+                ring_rhs[q] = res_load<RAGGED>(rhs_r + e, valid);
                 ring_den[q] = make_float4(inv_count((float)n), inv_count_lo((float)n), inv_count((float)end),
                                           inv_count_lo((float)end));
             }
@@ -203,8 +254,8 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
                 p[c][w][z] = zero4;
                 if (live) rhs[c * rcol + z * rplane + w * Wq] = zero4;
                 if ((w ? okB : okA) && k0 + z < g.D) {
-                    p[c][w][z] = *reinterpret_cast<const float4 *>((c ? p_b : p_r) + o);
-                    rhs[c * rcol + z * rplane + w * Wq] = ld4((c ? rhs_b : rhs_r) + o);
+                    p[c][w][z] = res_load<RAGGED>((c ? p_b : p_r) + o, lanes);
+                    rhs[c * rcol + z * rplane + w * Wq] = res_load<RAGGED>((c ? rhs_b : rhs_r) + o, lanes);
                     if (c == 1) sm[pcol + own + w * prow + z * pplane] = p[c][w][z];
                 }
             }
@@ -256,11 +307,16 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
                 }
                 const int n = cy[w] + cz[z];
                 const float2 in = inv[max(n, 0)], end = inv[max(n - (s == 0 ? c_lo : c_hi), 0)];
-                const QuadDen d = s == 0 ? QuadDen{end.y, end.x, in.y, in.x, in.y, in.x}
-                                         : QuadDen{in.y, in.x, in.y, in.x, end.y, end.x};
-                const float4 v = gs_quad_pk(sp.scale, s, rhs[c * rcol + z * rplane + w * Wq], x, xe,
-                                            w ? p[o][0][z] : ym, w ? yp : p[o][1][z], z ? p[o][w][z - 1] : zm[w],
-                                            z < RZ - 1 ? p[o][w][z + 1] : zp[w], d);
+                const float4 b = rhs[c * rcol + z * rplane + w * Wq], y0 = w ? p[o][0][z] : ym, y1 = w ? yp : p[o][1][z];
+                const float4 z0 = z ? p[o][w][z - 1] : zm[w], z1 = z < RZ - 1 ? p[o][w][z + 1] : zp[w];
+                float4 v;
+                if (RAGGED) {
+                    v = res_quad_ragged(sp.scale, s, b, x, xe, y0, y1, z0, z1, in, end, first, last, lanes);
+                } else {
+                    const QuadDen d = s == 0 ? QuadDen{end.y, end.x, in.y, in.x, in.y, in.x}
+                                             : QuadDen{in.y, in.x, in.y, in.x, end.y, end.x};
+                    v = gs_quad_pk(sp.scale, s, b, x, xe, y0, y1, z0, z1, d);
+                }
                 p[c][w][z] = v;
                 sc[w * prow + z * pplane] = v;
             }
@@ -277,8 +333,15 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
             const float4 *b = sm + pcol + at;
             const float4 n = ring_den[q];
             const float xe = cell & 2 ? 0.0f : reinterpret_cast<const float *>(b)[s ? 4 : -1];
-            const QuadDen d = s ? QuadDen{n.y, n.x, n.y, n.x, n.w, n.z} : QuadDen{n.w, n.z, n.y, n.x, n.y, n.x};
-            sm[at] = gs_quad(sp.scale, s, ring_rhs[q], *b, xe, b[-prow], b[prow], b[-pplane], b[pplane], d);
+            const float4 z0 = b[-pplane], z1 = b[pplane], y0 = b[-prow], y1 = b[prow];
+            if (RAGGED) {
+                const bool q_last = cell & 4;
+                sm[at] = res_quad_ragged(sp.scale, s, ring_rhs[q], *b, xe, y0, y1, z0, z1, make_float2(n.x, n.y),
+                                         make_float2(n.z, n.w), s == 0 && (cell & 2), s == 1 && q_last, q_last ? tail : 4);
+            } else {
+                const QuadDen d = s ? QuadDen{n.y, n.x, n.y, n.x, n.w, n.z} : QuadDen{n.w, n.z, n.y, n.x, n.y, n.x};
+                sm[at] = gs_quad(sp.scale, s, ring_rhs[q], *b, xe, y0, y1, z0, z1, d);
+            }
         }
     };
     // Exchanges: after every sweep but the last, whose black cells nobody reads
@@ -345,13 +408,15 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
 #pragma unroll
             for (int z = 0; z < RZ; ++z)
                 if ((w ? okB : okA) && k0 + z < g.D)
-                    *reinterpret_cast<float4 *>((c ? p_b : p_r) + gA + w * Wh + z * pl) = p[c][w][z];
+                    res_store<RAGGED>((c ? p_b : p_r) + gA + w * Wh + z * pl, p[c][w][z], lanes);
     if (threadIdx.x == 0) rs.epoch[blockIdx.x] = e0 + (unsigned)exchanges;
 }
 
 namespace {
 
 struct Shape { int RZ, NY, NZ, TY, TZ, threads; };
+
+int quads_of(const Geom &g) { return ((g.W >> 1) + 3) >> 2; }      // quads per packed row
 
 int sm_count() {
     static int cache[64] = {0};
@@ -376,8 +441,7 @@ size_t smem_of(int Wq, int TY, int TZ) {
 // The split of a grid over the SMs, one CTA each: the fewest cells per CTA
 // with its ring, then the smallest boundary.
 bool shape_of(const Geom &g, Shape *out) {
-    if ((g.W & 7) != 0) return false;
-    const int Wq = g.W >> 3, sms = sm_count();
+    const int Wq = quads_of(g), sms = sm_count();
     if (sms <= 0 || Wq > 256) return false;
     long long best = -1;
     for (int RZ = 2; RZ <= 4; RZ += 2) {
@@ -410,7 +474,7 @@ bool resident_supported(const Geom &g) {
 }
 
 static size_t halo_quads(const Geom &g, const Shape &s) {
-    return (size_t)s.NY * s.NZ * 4 * res_border(s.TY, s.TZ, g.W >> 3);
+    return (size_t)s.NY * s.NZ * 4 * res_border(s.TY, s.TZ, quads_of(g));
 }
 
 size_t resident_bytes(const Geom &g) {
@@ -423,14 +487,17 @@ cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *r
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st) {
     Shape s;
     if (!res.work || !res.err || sweeps < 1 || !shape_of(g, &s)) return cudaErrorInvalidValue;
-    const int ctas = s.NY * s.NZ, Wq = g.W >> 3;
+    const int ctas = s.NY * s.NZ, Wq = quads_of(g);
+    const bool ragged = (g.W & 7) != 0;
     ResParams rs{s.NY, s.NZ, s.TY, s.TZ, static_cast<uint4 *>(res.work), nullptr, res.err};
     rs.epoch = reinterpret_cast<unsigned *>(rs.halo + halo_quads(g, s));
     const size_t smem = smem_of(Wq, s.TY, s.TZ);
     const bool warprow = Wq <= 32 && 32 % Wq == 0 && (Wq * (s.TY / 2) * (s.TZ / s.RZ)) % 32 == 0;
     typedef void (*Kernel)(Geom, SolveParams, const float *, const float *, float *, float *, int, ResParams);
-    const Kernel k = s.RZ == 2 ? (warprow ? k_rbgs_resident<2, true> : k_rbgs_resident<2, false>)
-                               : (warprow ? k_rbgs_resident<4, true> : k_rbgs_resident<4, false>);
+    const Kernel k = s.RZ == 2 ? (ragged ? k_rbgs_resident<2, false, true> : warprow ? k_rbgs_resident<2, true, false>
+                                                                                    : k_rbgs_resident<2, false, false>)
+                               : (ragged ? k_rbgs_resident<4, false, true> : warprow ? k_rbgs_resident<4, true, false>
+                                                                                    : k_rbgs_resident<4, false, false>);
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};

@@ -2,7 +2,7 @@
 memory for a batch of sweeps, CTAs exchanging their borders.  They must give
 the segment kernel's bits (sweep variant 0) at every split of the grid: one
 CTA row or plane, ragged last CTAs, odd heights and depths, rows that straddle
-warps, one sweep (no exchange otherwise) and batches back to back."""
+warps, widths that are not whole quads, one sweep (no exchange otherwise) and batches back to back."""
 import numpy as np
 import pytest
 
@@ -29,7 +29,8 @@ def run(dims, variant, bc, batches):
 
 @pytest.mark.parametrize("dims", [(8, 4, 4), (8, 5, 7), (16, 4, 300), (8, 301, 6), (24, 21, 74), (40, 66, 59),
                                   (64, 64, 64), (120, 100, 84), (104, 40, 48), (200, 100, 60), (128, 128, 127),
-                                  (256, 40, 40), (384, 20, 61)])
+                                  (256, 40, 40), (384, 20, 61), (4, 4, 4), (6, 9, 5), (26, 151, 57),
+                                  (84, 64, 33), (90, 22, 36), (222, 82, 48)])
 @pytest.mark.parametrize("bc", [BLZ_BC_FREE_SURFACE, BLZ_BC_REF_COMPAT])
 def test_on_chip_sweeps_equal_segment_kernel(dims, bc):
     for batches in ((1,), (2,), (1, 3, 6)):
