@@ -1286,89 +1286,144 @@ void launch_reduce_pairs(const double *partials, int n, double *out2, cudaStream
 // pr/pb and delta in dr/db); each difference is formed as
 // (p0_a - p0_b) + (delta_a - delta_b), so the gradient keeps the correction's
 // digits that p0 + delta rounded to FP32 would lose.
+//
+// A thread takes the cells 2m and 2m + 1 of a row, one packed index of both
+// colours, through up to kGradPlanes planes, and updates the faces on their low
+// sides (and the domain's high faces in the last cells): V and W go as 8-byte
+// pairs, the z neighbour stays in registers, and every index is 32-bit
+// (blz_create refuses grids past that).  The bound is memory (p once, every face
+// read and written): 256^3 109 us, 4.3 TB/s, against 177 us with a thread per
+// cell and 64-bit offsets, which was bound by issue.
+constexpr int kGradPlanes = 8;
+constexpr int kGradBlocks = 148 * 8 * 2;       // eight blocks of 256 threads per SM
+
 template <bool DEFECT>
-__global__ void k_gradient(Geom g, SolveParams sp, float s, const float *__restrict__ pr,
-                           const float *__restrict__ pb, float *__restrict__ U,
-                           float *__restrict__ V, float *__restrict__ W, const float *__restrict__ dr,
-                           const float *__restrict__ db) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int j = blockIdx.y * blockDim.y + threadIdx.y;
-    const int k = blockIdx.z * blockDim.z + threadIdx.z;
-    if (i > g.W || j > g.H || k > g.D) return;
-    const int Wh = g.W >> 1, H = g.H;
+__global__ void __launch_bounds__(256)
+k_gradient(Geom g, SolveParams sp, float s, const float *__restrict__ pr, const float *__restrict__ pb,
+           float *__restrict__ U, float *__restrict__ V, float *__restrict__ W, const float *__restrict__ dr,
+           const float *__restrict__ db, int planes) {
+    const int m = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    const int Wh = g.W >> 1, H = g.H, D = g.D, pl = Wh * H, W2 = g.W;
+    const int k0 = blockIdx.z * planes, k1 = min(k0 + planes, D);
+    if (m >= Wh || j >= H) return;
     const OpenFaces &o = sp.open;
     const bool dir = sp.dirichlet;
-    auto P = [&](int a, int b, int c) { return pval(pr, pb, a, b, c, Wh, H); };
-    // p(a) - p(b), and p(a) alone (the difference to a Dirichlet ghost)
-    auto dP = [&](int a1, int b1, int c1, int a2, int b2, int c2) -> float {
-        if (DEFECT)
-            return (P(a1, b1, c1) - P(a2, b2, c2)) + (pval(dr, db, a1, b1, c1, Wh, H) - pval(dr, db, a2, b2, c2, Wh, H));
-        return P(a1, b1, c1) - P(a2, b2, c2);
-    };
-    auto P1 = [&](int a, int b, int c) -> float {
-        if (DEFECT) return (P(a, b, c) - 0.0f) + (pval(dr, db, a, b, c, Wh, H) - 0.0f);
-        return P(a, b, c) - 0.0f;
-    };
-    auto P1n = [&](int a, int b, int c) -> float {       // 0 - p(a)
-        if (DEFECT) return (0.0f - P(a, b, c)) + (0.0f - pval(dr, db, a, b, c, Wh, H));
-        return 0.0f - P(a, b, c);
-    };
-    if (j < g.H && k < g.D) {
-        const size_t q = lin(i, j, k, g.W + 1, g.H);
-        if (i > 0 && i < g.W) {
-            const float u = U[q] - s * dP(i, j, k, i - 1, j, k);
-            U[q] = u;
-            if (!dir && i == 1 && o.xlo) U[q - 1] = u;
-            if (!dir && i == g.W - 1 && o.xhi) U[q + 1] = u;
-        } else if (i == 0) {
-            if (!o.xlo) U[q] = 0.0f;
-            else if (dir) U[q] -= s * P1(0, j, k);
-        } else {
-            if (!o.xhi) U[q] = 0.0f;
-            else if (dir) U[q] -= s * P1n(g.W - 1, j, k);
+    // p (and delta) of the two cells
+    struct Pair { float a, b, da, db; };
+    auto at = [&](int e, bool odd) -> Pair {
+        Pair v{__ldg((odd ? pb : pr) + e), __ldg((odd ? pr : pb) + e), 0.0f, 0.0f};
+        if (DEFECT) {
+            v.da = __ldg((odd ? db : dr) + e);
+            v.db = __ldg((odd ? dr : db) + e);
         }
-    }
-    if (i < g.W && k < g.D) {
-        const size_t q = lin(i, j, k, g.W, g.H + 1);
-        const size_t row = (size_t)g.W;
-        if (j > 0 && j < g.H) {
-            const float v = V[q] - s * dP(i, j, k, i, j - 1, k);
-            V[q] = v;
-            if (!dir && j == 1 && o.ylo) V[q - row] = v;
-            if (!dir && j == g.H - 1 && o.yhi) V[q + row] = v;
-        } else if (j == 0) {
-            if (!o.ylo) V[q] = 0.0f;
-            else if (dir) V[q] -= s * P1(i, 0, k);
-        } else {
-            if (!o.yhi) V[q] = 0.0f;
-            else if (dir) V[q] -= s * P1n(i, g.H - 1, k);
+        return v;
+    };
+    auto diff = [&](float a, float da, float b, float db_) -> float {
+        return DEFECT ? (a - b) + (da - db_) : a - b;
+    };
+    int e = m + Wh * j + pl * k0;
+    int qu = 2 * m + (W2 + 1) * (j + H * k0), qv = 2 * m + W2 * (j + (H + 1) * k0), qw = 2 * (m + Wh * j + pl * k0);
+    bool odd = (j + k0) & 1;
+    Pair below{};
+    if (k0 > 0) below = at(e - pl, !odd);
+#pragma unroll 2
+    for (int k = k0; k < k1; ++k, odd = !odd, e += pl, qu += (W2 + 1) * H, qv += W2 * (H + 1), qw += 2 * pl) {
+        const Pair c = at(e, odd);
+        {   // U: the faces at 2m and 2m + 1
+            const float u1 = U[qu + 1] - s * diff(c.b, c.db, c.a, c.da);
+            U[qu + 1] = u1;
+            if (m > 0) {                                  // cell 2m - 1 has the colour of 2m + 1
+                const float x = __ldg((odd ? pr : pb) + e - 1), dx = DEFECT ? __ldg((odd ? dr : db) + e - 1) : 0.0f;
+                const float u0 = U[qu] - s * diff(c.a, c.da, x, dx);
+                U[qu] = u0;
+            } else if (!o.xlo) {
+                U[qu] = 0.0f;
+            } else {
+                U[qu] = dir ? U[qu] - s * diff(c.a, c.da, 0.0f, 0.0f) : u1;
+            }
+            if (m == Wh - 1) {
+                if (!o.xhi) U[qu + 2] = 0.0f;
+                else U[qu + 2] = dir ? U[qu + 2] - s * diff(0.0f, 0.0f, c.b, c.db) : u1;
+            }
         }
-    }
-    if (i < g.W && j < g.H) {
-        const size_t q = lin(i, j, k, g.W, g.H);
-        const size_t plane = (size_t)g.W * g.H;
-        if (k > 0 && k < g.D) {
-            const float w = W[q] - s * dP(i, j, k, i, j, k - 1);
-            W[q] = w;
-            if (!dir && k == 1 && o.zlo) W[q - plane] = w;
-            if (!dir && k == g.D - 1 && o.zhi) W[q + plane] = w;
-        } else if (k == 0) {
-            if (!o.zlo) W[q] = 0.0f;
-            else if (dir) W[q] -= s * P1(i, j, 0);
-        } else {
-            if (!o.zhi) W[q] = 0.0f;
-            else if (dir) W[q] -= s * P1n(i, j, g.D - 1);
+        {   // V
+            float2 *const q = reinterpret_cast<float2 *>(V + qv);
+            if (j > 0) {
+                const Pair y = at(e - Wh, !odd);
+                float2 v = *q;
+                v.x = v.x - s * diff(c.a, c.da, y.a, y.da);
+                v.y = v.y - s * diff(c.b, c.db, y.b, y.db);
+                *q = v;
+                if (!dir && j == 1 && o.ylo) *reinterpret_cast<float2 *>(V + qv - W2) = v;
+                if (!dir && j == H - 1 && o.yhi) *reinterpret_cast<float2 *>(V + qv + W2) = v;
+            } else if (!o.ylo) {
+                *q = make_float2(0.0f, 0.0f);
+            } else if (dir) {
+                float2 v = *q;
+                v.x -= s * diff(c.a, c.da, 0.0f, 0.0f);
+                v.y -= s * diff(c.b, c.db, 0.0f, 0.0f);
+                *q = v;
+            }
+            if (j == H - 1) {
+                float2 *const h = reinterpret_cast<float2 *>(V + qv + W2);
+                if (!o.yhi) {
+                    *h = make_float2(0.0f, 0.0f);
+                } else if (dir) {
+                    float2 v = *h;
+                    v.x -= s * diff(0.0f, 0.0f, c.a, c.da);
+                    v.y -= s * diff(0.0f, 0.0f, c.b, c.db);
+                    *h = v;
+                }
+            }
         }
+        {   // W
+            float2 *const q = reinterpret_cast<float2 *>(W + qw);
+            if (k > 0) {
+                float2 v = *q;
+                v.x = v.x - s * diff(c.a, c.da, below.a, below.da);
+                v.y = v.y - s * diff(c.b, c.db, below.b, below.db);
+                *q = v;
+                if (!dir && k == 1 && o.zlo) *reinterpret_cast<float2 *>(W + qw - 2 * pl) = v;
+                if (!dir && k == D - 1 && o.zhi) *reinterpret_cast<float2 *>(W + qw + 2 * pl) = v;
+            } else if (!o.zlo) {
+                *q = make_float2(0.0f, 0.0f);
+            } else if (dir) {
+                float2 v = *q;
+                v.x -= s * diff(c.a, c.da, 0.0f, 0.0f);
+                v.y -= s * diff(c.b, c.db, 0.0f, 0.0f);
+                *q = v;
+            }
+            if (k == D - 1) {
+                float2 *const h = reinterpret_cast<float2 *>(W + qw + 2 * pl);
+                if (!o.zhi) {
+                    *h = make_float2(0.0f, 0.0f);
+                } else if (dir) {
+                    float2 v = *h;
+                    v.x -= s * diff(0.0f, 0.0f, c.a, c.da);
+                    v.y -= s * diff(0.0f, 0.0f, c.b, c.db);
+                    *h = v;
+                }
+            }
+        }
+        // the planes above have it as their lower neighbour; the cells' colours
+        // swap with the plane, the pair's order does not
+        below = c;
     }
 }
 
 void launch_gradient(const Geom &g, const SolveParams &sp, float s, const float *p_r,
                      const float *p_b, float *U, float *V, float *W, cudaStream_t st, const float *d_r,
                      const float *d_b) {
+    const dim3 blk(32, 8);
+    const unsigned bx = ((g.W >> 1) + blk.x - 1) / blk.x, by = (g.H + blk.y - 1) / blk.y;
+    // Enough blocks to fill the chip twice before a thread takes more planes.
+    int planes = kGradPlanes;
+    while (planes > 1 && (long long)bx * by * ((g.D + planes - 1) / planes) < kGradBlocks) planes >>= 1;
+    const dim3 grid(bx, by, (g.D + planes - 1) / planes);
     if (d_r && d_b)
-        k_gradient<true><<<face_grid(g), face_block(), 0, st>>>(g, sp, s, p_r, p_b, U, V, W, d_r, d_b);
+        k_gradient<true><<<grid, blk, 0, st>>>(g, sp, s, p_r, p_b, U, V, W, d_r, d_b, planes);
     else
-        k_gradient<false><<<face_grid(g), face_block(), 0, st>>>(g, sp, s, p_r, p_b, U, V, W, nullptr, nullptr);
+        k_gradient<false><<<grid, blk, 0, st>>>(g, sp, s, p_r, p_b, U, V, W, nullptr, nullptr, planes);
 }
 
 // The defect of the current pressure for the defect-correction solve, in
