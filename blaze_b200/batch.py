@@ -58,8 +58,9 @@ class Batch:
         """-1: autotune (default); 0: the segment kernel; planes > 0: temporal
         blocking with tiles of that many planes (paired: the paired-FP32
         stencil).  Every choice gives the same bits; the stats' sweep_variant
-        reports the one in use (1, 2, 4, 8 planes per thread, or 100 (scalar)
-        or 200 (paired) + planes per tile)."""
+        reports the one in use (1, 2, 4, 8 planes per thread, 100 (scalar) or
+        200 (paired) + planes per tile, or 11: on chip, which the autotuner
+        tries where every grid fits)."""
         check(self._lib.blz_batch_set_sweep(self._h, int(planes), 1 if paired else 0))
 
     def last_ms(self):

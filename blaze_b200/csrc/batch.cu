@@ -12,7 +12,8 @@
 // {check_every sweeps, residual, decision} until no grid is left running.
 // Each grid stops exactly where its own device-loop solve stops, with the
 // same pressure bit for bit.  The launch shape (planes per thread and block
-// size) is autotuned per batch on scratch copies of the pressures.
+// size, temporal-blocking tiles, or the on-chip sweeps of several grids side by
+// side) is autotuned per batch on scratch copies of the pressures.
 //
 // When no grid's forces depend on time (no curl noise, no moving wind
 // noise), a whole frame — every grid's forces and divergence, the batched
@@ -22,6 +23,7 @@
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
+#include <cstdlib>
 #include <string>
 #include <vector>
 
@@ -89,6 +91,12 @@ struct blz_batch {
     BatchTile *d_tiles = nullptr;             // tiles of the current tb_zc, heaviest first
     int ntiles = 0, tiles_cap = 0;
     size_t tb_smem = 0;                       // largest dynamic shared memory of a tile
+    // on-chip sweeps: waves of grids (empty: a grid does not fit), their
+    // exchange buffers and error flag
+    std::vector<ResidentWave> waves;
+    void *res_work = nullptr;
+    int *res_err = nullptr;
+    bool on_chip = false;                     // chosen
     bool time_free = false;                   // frame graphs allowed
     cudaGraphExec_t solve_exec = nullptr;
     cudaGraphExec_t frame_exec[2] = {nullptr, nullptr};
@@ -171,12 +179,19 @@ static int build_tiles(blz_batch *b, const std::vector<BatchSim> &h, int zc) {
 
 // Body of the batched solve, appended to the capture in progress on b->st:
 // check_every sweeps over the grids still running, their residual and decision.
-static void capture_body(blz_batch *b, cudaGraphConditionalHandle h) {
-    if (b->tb_zc > 0)
+static cudaError_t capture_body(blz_batch *b, cudaGraphConditionalHandle h) {
+    cudaError_t e = cudaSuccess;
+    if (b->on_chip) e = launch_batch_resident(b->waves, b->d_ctl, b->chunk, b->st);
+    else if (b->tb_zc > 0)
         launch_batch_tb(b->d_sims, b->d_tiles, b->ntiles, b->d_ctl, b->chunk, b->tb_smem, b->tb_pk, b->st);
     else launch_batch_sweeps(b->d_sims, b->d_act, b->n, b->chunk, b->kz, b->grid, b->block, b->st);
     launch_batch_check(b->d_sims, b->d_blk0, b->n, b->total_blocks, b->d_ctl, b->partials, 1, b->chunk, b->st);
     active_list(b, b->kz, 1, h);
+    return e;
+}
+
+static int body_launches(const blz_batch *b) {
+    return (b->on_chip ? (int)b->waves.size() : b->tb_zc > 0 ? b->chunk / 2 : 2 * b->chunk) + 2 + 1;
 }
 
 // Builds [stages before the solve] + solve loop + [stages after] as one graph.
@@ -240,10 +255,11 @@ static int build_graph(blz_batch *b, bool with_stages, cudaGraphExec_t *out, lon
     if (e != cudaSuccess || rc != BLZ_OK) goto done;
     e = cudaStreamBeginCaptureToGraph(b->st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) goto done;
-    capture_body(b, h);
     {
+        const cudaError_t launched = capture_body(b, h);
         cudaGraph_t g2 = nullptr;
         e = cudaStreamEndCapture(b->st, &g2);
+        if (e == cudaSuccess) e = launched;
     }
     if (e != cudaSuccess) goto done;
     if (with_stages) {
@@ -276,9 +292,11 @@ done:
 
 // Autotuner: the segment kernel's planes per thread x block size (two sweeps
 // of the whole batch timed) against temporal blocking with 8, 16 or 32
-// planes per tile, scalar or paired-FP32 stencil (four sweeps timed), per
-// sweep, on scratch copies of every pressure (all shapes give identical
-// results).
+// planes per tile, scalar or paired-FP32 stencil (four sweeps timed) and, where
+// every grid fits, the on-chip sweeps (one check interval timed, 20 sweeps at
+// most), per sweep, on scratch copies of every pressure (all shapes give
+// identical results).  BLZ_SWEEP_VARIANT naming the on-chip sweeps makes them
+// the choice where every grid fits, as for one solver.
 static int tune(blz_batch *b) {
     if (b->kz >= 0) return BLZ_OK;
     std::vector<BatchSim> h(b->n), hs(b->n);
@@ -341,6 +359,27 @@ static int tune(blz_batch *b) {
             if (e == cudaSuccess && ms / 4.0f < best) { best = ms / 4.0f; tb_best = zc; pk_best = pk != 0; }
         }
     }
+    b->on_chip = false;
+    if (!b->waves.empty() && b->force_zc < 0 && e == cudaSuccess) {
+        std::vector<ResidentWave> w = b->waves;
+        for (auto &x : w)
+            for (int i = 0; i < x.n; ++i) {
+                x.grid[i].p_r = hs[x.grid[i].sim].p_r;
+                x.grid[i].p_b = hs[x.grid[i].sim].p_b;
+            }
+        const int timed = std::min(b->chunk, 20);
+        e = launch_batch_resident(w, b->d_ctl, timed, b->st);
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev0, b->st);
+        if (e == cudaSuccess) e = launch_batch_resident(w, b->d_ctl, timed, b->st);
+        if (e == cudaSuccess) e = cudaEventRecord(b->ev1, b->st);
+        if (e == cudaSuccess) e = cudaEventSynchronize(b->ev1);
+        float ms = 0.0f;
+        if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, b->ev0, b->ev1);
+        b->launches += 2 * (long long)w.size();
+        const char *env = std::getenv("BLZ_SWEEP_VARIANT");
+        b->on_chip = e == cudaSuccess && (ms / timed < best || (env && std::atoi(env) == kResidentVariant));
+        if (b->on_chip) tb_best = 0;
+    }
     if (e == cudaSuccess && tb_best > 0) {
         b->tb_zc = tb_best;
         b->tb_pk = pk_best;
@@ -364,6 +403,8 @@ static void release(blz_batch *b) {
     cudaFree(b->d_sims); cudaFree(b->d_ctl); cudaFree(b->d_item0); cudaFree(b->d_blk0); cudaFree(b->partials);
     cudaFree(b->d_act); cudaFree(b->d_act_sim); cudaFree(b->d_act_item0); cudaFree(b->d_tiles);
     if (b->h_ctl) cudaFreeHost(b->h_ctl);
+    if (b->res_err) cudaFreeHost(b->res_err);
+    cudaFree(b->res_work);
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     if (b->st) cudaStreamDestroy(b->st);
@@ -372,6 +413,10 @@ static void release(blz_batch *b) {
 static int read_stats(blz_batch *b, blz_step_stats *stats, int loop_ran) {
     BCK(cudaMemcpyAsync(b->h_ctl, b->d_ctl, sizeof(BatchCtl) * b->n, cudaMemcpyDeviceToHost, b->st));
     BCK(cudaStreamSynchronize(b->st));
+    if (b->res_err && *b->res_err) {
+        *b->res_err = 0;
+        return bfail(BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up");
+    }
     for (int i = 0; i < b->n; ++i)
         if (blz_unet *u = solver_warm(b->sims[i])) {
             const int rc = unet_timeout_flag(u, b->st);
@@ -394,7 +439,7 @@ static int read_stats(blz_batch *b, blz_step_stats *stats, int loop_ran) {
         st.rhs_norm = bn;
         st.rel_residual = bn > 0.0 ? r / bn : 0.0;
         st.residual_checks = c.checks;
-        st.sweep_variant = b->tb_zc > 0 ? (b->tb_pk ? 200 : 100) + b->tb_zc : b->kz;
+        st.sweep_variant = b->on_chip ? kResidentVariant : b->tb_zc > 0 ? (b->tb_pk ? 200 : 100) + b->tb_zc : b->kz;
         st.device_loop = 1;
         if (solver_warm(b->sims[i])) {
             st.warm_started = 1;
@@ -488,6 +533,16 @@ int blz_batch_create(blz_solver *const *sims, int n, blz_batch **out) {
     if (rc == BLZ_OK) ck(cudaMemcpy(b->d_item0, item0.data(), sizeof(long long) * item0.size(), cudaMemcpyHostToDevice), "cudaMemcpy");
     if (rc == BLZ_OK) ck(cudaMemcpy(b->d_blk0, blk0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice), "cudaMemcpy");
     for (int i = 0; i < n && rc == BLZ_OK; ++i) rc = blz_set_stream(sims[i], b->st);
+    size_t res_bytes = 0;
+    if (rc == BLZ_OK && batch_resident_plan(h.data(), n, &b->waves, &res_bytes)) {
+        ck(cudaMalloc(&b->res_work, res_bytes), "cudaMalloc");
+        if (rc == BLZ_OK) ck(cudaMemset(b->res_work, 0, res_bytes), "cudaMemset");
+        if (rc == BLZ_OK) ck(cudaMallocHost(&b->res_err, sizeof(int)), "cudaMallocHost");
+        if (rc == BLZ_OK) {
+            *b->res_err = 0;
+            batch_resident_bind(&b->waves, b->res_work, b->res_err);
+        }
+    }
     b->prologue = 1 + 2 + 1;                 // begin, residual + decision, active list
     if (rc != BLZ_OK) {
         release(b);
@@ -546,7 +601,7 @@ int blz_batch_solve(blz_batch *b, blz_step_stats *stats) {
     if (!b) return bfail(BLZ_ERR_ARG, "null batch");
     int rc = tune(b);
     if (rc != BLZ_OK) return rc;
-    b->body = (b->tb_zc > 0 ? b->chunk / 2 : 2 * b->chunk) + 2 + 1;
+    b->body = body_launches(b);
     if (!b->solve_exec && (rc = build_solve_graph_of(b)) != BLZ_OK) return rc;
     BCK(cudaEventRecord(b->ev0, b->st));
     BCK(cudaGraphLaunch(b->solve_exec, b->st));
@@ -561,7 +616,7 @@ int blz_batch_step(blz_batch *b, const float *times, blz_step_stats *stats) {
     if (!b) return bfail(BLZ_ERR_ARG, "null batch");
     int rc = tune(b);
     if (rc != BLZ_OK) return rc;
-    b->body = (b->tb_zc > 0 ? b->chunk / 2 : 2 * b->chunk) + 2 + 1;
+    b->body = body_launches(b);
     if (b->time_free) {
         const int par = b->parity;
         if (!b->frame_exec[par]) {

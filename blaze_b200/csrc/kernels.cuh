@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda.h>   // CUtensorMap and its enums (the encoder comes from cudaGetDriverEntryPoint)
 #include <cuda_runtime.h>
+#include <vector>
 
 #include "common.cuh"
 
@@ -228,6 +229,31 @@ int  batch_tb_rows(const Geom &g);
 size_t batch_tb_smem(const Geom &g);
 void launch_batch_tb(const BatchSim *sims, const BatchTile *tiles, int ntiles, const BatchCtl *ctl, int sweeps,
                      size_t smem, bool pk, cudaStream_t st);
+// The on-chip sweeps in a batch (k_resident.cu): waves of up to kWaveGrids grids,
+// one cooperative launch each, grid i on CTAs [cta0, cta0 + NY * NZ).  plan:
+// false where a grid does not fit; else the waves, their exchange buffers as
+// offsets into `bytes` of device memory, zeroed once, which bind adds with the
+// error flag (mapped host memory, set nonzero when a wait gave up).
+constexpr int kWaveGrids = 16;
+struct ResidentGrid {
+    Geom g;
+    SolveParams sp;
+    const float *rhs_r, *rhs_b;
+    float *p_r, *p_b;
+    void *halo;
+    unsigned *epoch;
+    int NY, NZ, TY, TZ, sim, cta0, warprow;
+};
+struct ResidentWave {
+    ResidentGrid grid[kWaveGrids];
+    int n, ctas, RZ;
+    size_t smem;
+    int *err;
+};
+static_assert(sizeof(ResidentWave) <= 4000, "a wave travels as a kernel argument");
+bool batch_resident_plan(const BatchSim *sims, int n, std::vector<ResidentWave> *waves, size_t *bytes);
+void batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err);
+cudaError_t launch_batch_resident(const std::vector<ResidentWave> &waves, const BatchCtl *ctl, int sweeps, cudaStream_t st);
 // FP64 residual of every active grid (grid s owns partial blocks
 // [blk0[s], blk0[s+1]), residual_blocks(g_s) of them) and the per-grid
 // continue/stop decision.  2 launches.

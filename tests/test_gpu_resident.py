@@ -2,7 +2,8 @@
 memory for a batch of sweeps, CTAs exchanging their borders.  They must give
 the segment kernel's bits (sweep variant 0) at every split of the grid: one
 CTA row or plane, ragged last CTAs, odd heights and depths, rows that straddle
-warps, widths that are not whole quads, one sweep (no exchange otherwise) and batches back to back."""
+warps, widths that are not whole quads, one sweep (no exchange otherwise) and
+batches back to back."""
 import numpy as np
 import pytest
 
@@ -53,3 +54,49 @@ def test_on_chip_solve_counts_and_reports():
                 assert st["sweep_variant"] == ON_CHIP and st["device_loop"] == 1
     assert out[0][:2] == out[1][:2]
     np.testing.assert_array_equal(out[0][2], out[1][2])
+
+
+BATCHES = {
+    "one wave": [(16, 16, 16), (64, 96, 40), (48, 40, 31), (8, 4, 5)],
+    "several waves": [(128, 64, 64), (96, 96, 96), (384, 20, 61), (64, 64, 64), (8, 301, 6), (128, 128, 128), (48, 47, 48)],
+    "many small": [(8 + 8 * (i % 3), 5 + i, 4 + (7 * i) % 11) for i in range(19)],
+}
+
+
+@pytest.mark.parametrize("name", BATCHES)
+@pytest.mark.parametrize("check_every", [1, 10])
+def test_on_chip_batch_equals_single_solves(name, check_every, monkeypatch):
+    """Grids swept side by side, in one or several launches, while some have
+    already stopped: each grid's sweep count, residual and pressure are those
+    of its own solve with the segment kernel, bit for bit."""
+    from blaze_b200 import FluidSolver, Timer
+    from blaze_b200.batch import Batch
+    from blaze_b200.scenes import SceneSettings
+    monkeypatch.setenv("BLZ_SWEEP_VARIANT", "11")
+    runs = []
+    for batched in (False, True):
+        sims = []
+        for i, d in enumerate(BATCHES[name]):
+            rng = np.random.default_rng(70 + i)
+            W, H, D = d
+            sims.append(FluidSolver(Timer(), SceneSettings(
+                gridRes=d, dx=1 / 64, closedBounds=(1, 1, 1, 0, 1, 1), bc_mode=BLZ_BC_FREE_SURFACE, sweep_variant=0,
+                maxIterSolve=60, tol=(0.2, 0.02, 1e-3)[i % 3], check_every=check_every)))
+            sims[-1].set("RHS", rng.standard_normal((D, H, W)).astype(np.float32))
+        if batched:
+            batch = Batch(sims)
+            stats = [batch.solve(), batch.solve()]
+            assert all(st["sweep_variant"] == 11 for st in stats[0])
+            batch.close()
+        else:
+            stats = [[s.solve() for s in sims] for _ in range(2)]
+        runs.append((stats, [s.get("P") for s in sims]))
+        for s in sims:
+            s.close()
+    (sa, pa), (sb, pb) = runs
+    for f in range(2):
+        for i in range(len(pa)):
+            assert sa[f][i]["iterations"] == sb[f][i]["iterations"], (f, i)
+            assert sa[f][i]["residual"] == sb[f][i]["residual"], (f, i)
+    for i in range(len(pa)):
+        assert np.array_equal(pa[i], pb[i]), i
