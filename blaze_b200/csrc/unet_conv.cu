@@ -235,9 +235,7 @@ k_conv3d_tc(int W, int H, int D, int cin, int out_stride, int out_offset, const 
 int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 
 // ---------------------------------------------------------------------------
-// z-marching variant for the layers with 16 to 64 input and output channels
-// whose weights fit in shared memory (they carry nearly all of the network's
-// voxels).  A CTA keeps the layer's weights resident and walks a tile of 8 x 16
+// z-marching variant for the layers of 16 to 128 input and output channels.  A CTA keeps the layer's weights resident and walks a tile of 8 x 16
 // voxels (x, y) through `zs` output planes.
 //
 // What bounds such a layer is the number of MMAs: with 16 output channels one
@@ -265,9 +263,15 @@ int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 // their next wait; before the CTA ends, the MMA warp waits for its last commit
 // and the copy warp for every copy it issued.
 //
+// Layers whose weights do not fit (64 or 128 channels in, 64 or 128 out) are cut
+// by output channels: a CTA takes N of them, so the input is staged cout / N
+// times, mostly from L2.
+//
 // Measured (16 -> 16 at 256^3, 32 -> 16 at 256^3, 32 -> 32 at 128^3, 64 -> 32 at
 // 128^3): 461, 786, 139 and 360 us; with an MMA per tap and output plane on 128
-// voxels of a row 738, 1994, 298 and (general kernel) 1146 us.  What bounds it
+// voxels of a row 738, 1994, 298 and (general kernel) 1146 us.  By parts, 64 ->
+// 64 and 128 -> 64 at 64^3, 64 -> 128 and 128 -> 128 at 32^3: 100, 325, 35 and 96
+// us (general kernel about 228, 456, 62 and 124).  What bounds it
 // now: the copies, whose innermost run is 16 bytes (344 us of the 461 remain
 // without the MMAs and the epilogue), then the MMAs.
 // ---------------------------------------------------------------------------
@@ -287,7 +291,7 @@ template <int N, int CIN> struct Zm {
     static constexpr int kWeights = 27 * CH * N * 32;
     // output planes in flight: 3 for a plane's own MMAs, 2 per later chunk, and
     // at least 3 being read out; a power of two
-    static constexpr int R = 2 * (CH - 1) + 6 <= 8 ? 8 : 16;
+    static constexpr int R = 2 * (CH - 1) + 6 <= 8 ? 8 : 2 * (CH - 1) + 6 <= 16 ? 16 : 32;
     static constexpr int kCols = R * N;
     static constexpr bool kTwo = kCols <= 256 && kWeights + 128 + 6 * kZmBlock <= kZmSmemTwo;   // CTAs per SM
     static constexpr int kRoom = ((kTwo ? kZmSmemTwo : kZmSmemOne) - kWeights - 128) / kZmBlock;
@@ -313,7 +317,8 @@ __device__ __forceinline__ void zm_commit(uint32_t lead, uint32_t bar) {
 
 template <int N, int CIN, bool RELU>
 __global__ void __launch_bounds__(kZmThreads, 1)
-k_conv3d_zm(int W, int H, int D, int zs, int out_stride, int out_offset, const __grid_constant__ CUtensorMap xmap,
+k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offset,
+            const __grid_constant__ CUtensorMap xmap,
             const __nv_bfloat16 *__restrict__ w, const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y,
             const __nv_bfloat16 *__restrict__ aux, int *err) {
     extern __shared__ __align__(128) unsigned char smem[];
@@ -324,7 +329,11 @@ k_conv3d_zm(int W, int H, int D, int zs, int out_stride, int out_offset, const _
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int Wp = W + 2, Hp = H + 2;
-    const int X0 = blockIdx.x * kZmTX, Y0 = blockIdx.y * kZmTY, z0 = blockIdx.z * zs;
+    const int part = blockIdx.z % parts, cout = parts * N;      // this CTA's output channels: part N .. part N + N - 1
+    const int X0 = blockIdx.x * kZmTX, Y0 = blockIdx.y * kZmTY, z0 = (int)(blockIdx.z / parts) * zs;
+    w += (size_t)part * N * CIN;
+    if (bias) bias += part * N;
+    out_offset += part * N;
     const int nz = (z0 + zs < D ? z0 + zs : D) - z0;
 
     if (warp == 0) {
@@ -349,7 +358,7 @@ k_conv3d_zm(int W, int H, int D, int zs, int out_stride, int out_offset, const _
         const int kg = e & 1, n = (e >> 1) % N, ct = (e >> 1) / N;          // ct = ch * 27 + tap
         const int ch = ct / 27, t = ct % 27, o = 2 - t / 9, t9 = t % 9;
         cp_async16(bS + (ch * 9 + t9) * kTap + kg * 3 * N * 16 + (o * N + n) * 16,
-                   w + ((size_t)t * N + n) * CIN + ch * 16 + kg * 8);
+                   w + ((size_t)t * cout + n) * CIN + ch * 16 + kg * 8);
     }
     asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -558,7 +567,8 @@ static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const _
     if (!zm_tensor_map(&xm, x, cd)) return cudaErrorNotSupported;
     // Output planes per CTA: the least time of a whole number of waves, a CTA of
     // zs planes taking zs + 2 + 2 (CH - 1) rounds and about 6 more to start.
-    const long long tiles = (long long)((cd.W + kZmTX - 1) / kZmTX) * ((cd.H + kZmTY - 1) / kZmTY);
+    const int parts = cd.cout / N;
+    const long long tiles = (long long)((cd.W + kZmTX - 1) / kZmTX) * ((cd.H + kZmTY - 1) / kZmTY) * parts;
     const long long room = (long long)conv_sm_count() * (Z::kTwo ? 2 : 1);
     int zs = 0;
     long long best = 0;
@@ -567,9 +577,9 @@ static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const _
         if (zs == 0 || cost < best) { zs = v; best = cost; }
     }
     const dim3 grid((unsigned)((cd.W + kZmTX - 1) / kZmTX), (unsigned)((cd.H + kZmTY - 1) / kZmTY),
-                    (unsigned)((cd.D + zs - 1) / zs));
+                    (unsigned)(parts * ((cd.D + zs - 1) / zs)));
     const int os = cd.out_stride > 0 ? cd.out_stride : cd.cout;
-    k_conv3d_zm<N, CIN, RELU><<<grid, kZmThreads, Z::kSmem, st>>>(cd.W, cd.H, cd.D, zs, os, cd.out_offset, xm, w, bias,
+    k_conv3d_zm<N, CIN, RELU><<<grid, kZmThreads, Z::kSmem, st>>>(cd.W, cd.H, cd.D, zs, parts, os, cd.out_offset, xm, w, bias,
                                                                   static_cast<__nv_bfloat16 *>(y), aux, err);
     return cudaGetLastError();
 }
@@ -579,18 +589,23 @@ static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const _
 static bool zm_dispatch(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
                         void *y, const __nv_bfloat16 *aux, int *err, cudaStream_t st, cudaError_t *res) {
     if (cd.out_f32) return false;
-#define BLZ_ZM(NN, CC)                                                                              \
-    if (cd.cout == NN && cd.cin == CC) {                                                            \
+#define BLZ_ZM(OUT, NN, CC)                                                                         \
+    if (cd.cout == OUT && cd.cin == CC) {                                                           \
         *res = cd.relu ? launch_zm<NN, CC, true>(cd, x, w, bias, y, aux, err, st)                   \
                        : launch_zm<NN, CC, false>(cd, x, w, bias, y, aux, err, st);                 \
         return true;                                                                                \
     }
-    BLZ_ZM(16, 16)
-    BLZ_ZM(16, 32)
-    BLZ_ZM(32, 16)
-    BLZ_ZM(32, 32)
-    BLZ_ZM(32, 64)
-    BLZ_ZM(64, 32)
+    BLZ_ZM(16, 16, 16)
+    BLZ_ZM(16, 16, 32)
+    BLZ_ZM(32, 32, 16)
+    BLZ_ZM(32, 32, 32)
+    BLZ_ZM(32, 32, 64)
+    BLZ_ZM(64, 64, 32)
+    // weights past shared memory: by parts of the output channels
+    BLZ_ZM(64, 32, 64)
+    BLZ_ZM(128, 32, 64)
+    BLZ_ZM(64, 16, 128)
+    BLZ_ZM(128, 16, 128)
 #undef BLZ_ZM
     return false;
 }

@@ -70,6 +70,15 @@ def test_conv3d_tensor_cores(shape, cin, cout, relu, out_f32):
     assert float(yv[0].abs().max()) == 0.0 and float(yv[:, :, 0].abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("shape,cin,cout,relu", [
+    ((5, 3, 1), 128, 128, True), ((9, 17, 2), 64, 128, False), ((8, 16, 33), 128, 64, True),
+    ((23, 18, 19), 64, 64, False), ((17, 5, 65), 128, 128, False)])
+def test_conv3d_by_output_channels(shape, cin, cout, relu):
+    """Layers cut by output channels: one plane, fewer planes than chunks,
+    several z slabs, ragged tiles."""
+    test_conv3d_tensor_cores(shape, cin, cout, relu, 0)
+
+
 # ---------------------------------------------------------------------------
 # The whole warm-start network against the FP64 oracle with BF16 rounding
 # emulated at the GPU's storage points (oracle/unet_oracle.py).  Each
