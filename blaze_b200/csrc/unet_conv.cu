@@ -16,6 +16,8 @@
 // A operand of tap (dx, dy, dz) is the same block seen 16*(dx+1) B further
 // on: 27 MMAs of M=128 x N x K=16 read one staged block.  The halo makes
 // the zero padding of the convolution a plain memory read.
+#include <algorithm>
+
 #include <cuda_bf16.h>
 
 #include "kernels.cuh"
@@ -659,25 +661,57 @@ cudaError_t launch_conv3d(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv
 // MMAs and commits them to an mbarrier (bounded wait); the epilogue reads
 // each parity's COUT columns from TMEM, adds the bias and stores BF16 into
 // the fine voxel's channels [0, COUT) of a tensor with channel stride ys.
+//
+// Persistent: as many CTAs as the SMs' tensor memory holds, the weights staged
+// once each and the next tile's voxels while this one's are read out.  What
+// bounds it is the output, 16 channels of 32 (with the skip half) per fine voxel
+// at 256^3, whose 32-byte sectors one store fills.  32 -> 16 to 256^3 196 us, 64 ->
+// 32 to 128^3 54, 128 -> 64 to 64^3 21; a CTA per tile that staged, multiplied and
+// read out in turn, with 16-byte stores: 390, 106 and 37.
 // ---------------------------------------------------------------------------
+template <int CIN, int COUT> struct UpShape {
+    static constexpr int N = 8 * COUT, CH = CIN / 16;
+    static constexpr int kAChunk = 2 * kConvM * 16;      // [kg][voxel][8] of one 16-channel chunk
+    static constexpr int kBChunk = 2 * N * 16;           // [kg][n][8] of one 16-channel chunk
+    static constexpr int kABytes = CH * kAChunk;
+    static constexpr int SMEM = 2 * kABytes + CH * kBChunk;
+    static constexpr int kPerSm = 512 / N;               // CTAs an SM's tensor memory holds
+    static_assert(kPerSm * (SMEM + 1024) <= 227 * 1024, "shared memory for as many");
+};
+
+// 16 BF16 outputs of a voxel: one 32-byte store, which fills its sector, where
+// the tensor's layout allows it.
+__device__ __forceinline__ void st_bf16x16(__nv_bfloat16 *dst, const uint32_t v[8], bool wide) {
+    if (wide) {
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                     ::"l"(dst), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                     : "memory");
+    } else {
+        reinterpret_cast<uint4 *>(dst)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+        reinterpret_cast<uint4 *>(dst)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+    }
+}
+static bool wide_stores(const void *y, int stride, int offset) {
+    return (reinterpret_cast<uintptr_t>(y) & 31) == 0 && stride % 16 == 0 && offset % 16 == 0;
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(128, 1)
 k_upconv_tc(int W, int H, int D, const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w,
-            const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y, int ys, int *err) {
-    constexpr int N = 8 * COUT, CH = CIN / 16;
+            const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y, int ys, int wide, int *err) {
+    typedef UpShape<CIN, COUT> S;
+    constexpr int N = S::N, CH = S::CH, kAChunk = S::kAChunk, kBChunk = S::kBChunk;
     constexpr int NMMA = N > 256 ? 256 : N;              // columns per MMA
     constexpr int kCols = N;                              // 128, 256 or 512: a power of two
-    constexpr int kAChunk = 2 * kConvM * 16;              // [kg][voxel][8] of one 16-channel chunk
-    constexpr int kBChunk = 2 * N * 16;                   // [kg][n][8] of one 16-channel chunk
     constexpr uint32_t idesc = umma_idesc_bf16(kConvM, NMMA);
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t mbar;
+    __shared__ __align__(16) float sbias[COUT];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int Wp = W + 2, Hp = H + 2;
     const long long plane = (long long)Wp * Hp;
-    const int z = blockIdx.y;                                              // interior coarse plane
-    const long long P0 = (long long)Wp + (long long)kConvM * blockIdx.x;   // first voxel of the tile
+    const int tiles_x = (Wp * H + kConvM - 1) / kConvM, tiles = tiles_x * D;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
@@ -688,96 +722,121 @@ k_upconv_tc(int W, int H, int D, const __nv_bfloat16 *__restrict__ x, const __nv
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(&mbar)) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem = tmem_base;
-    const uint32_t aS = smem_u32(smem), bS = aS + (uint32_t)(CH * kAChunk);
-    // A: 16-byte chunk (c, kg) of voxel v at aS + c kAChunk + kg 2048 + v 16.
-    const __nv_bfloat16 *xs = x + ((long long)(z + 1) * plane + P0) * CIN;
-    for (int e = tid; e < CH * 2 * kConvM; e += 128) {
-        const int c = e / (2 * kConvM), r = e % (2 * kConvM), kg = r & 1, v = r >> 1;
-        cp_async16(aS + c * kAChunk + kg * (kConvM * 16) + v * 16, xs + (long long)v * CIN + c * 16 + kg * 8);
-    }
+    for (int e = tid; e < COUT; e += 128) sbias[e] = bias[e];
+    const uint32_t aS = smem_u32(smem), bS = aS + (uint32_t)(2 * S::kABytes);
+    // Tile t: 128 voxels of interior coarse plane t / tiles_x.  A: 16-byte chunk
+    // (c, kg) of voxel v at c kAChunk + kg 2048 + v 16.
+    auto stage = [&](int t, uint32_t dst) {
+        const int z = t / tiles_x;
+        const __nv_bfloat16 *xs = x + ((long long)(z + 1) * plane + Wp + (long long)kConvM * (t - z * tiles_x)) * CIN;
+        for (int e = tid; e < CH * 2 * kConvM; e += 128) {
+            const int kc = e % (2 * CH), v = e / (2 * CH);      // a voxel's chunks side by side: whole lines
+            cp_async16(dst + (kc >> 1) * kAChunk + (kc & 1) * (kConvM * 16) + v * 16, xs + (long long)v * CIN + kc * 8);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     // B: 16-byte chunk (c, kg) of row n at bS + c kBChunk + kg N 16 + n 16.
     for (int e = tid; e < CH * 2 * N; e += 128) {
         const int c = e / (2 * N), r = e % (2 * N), kg = r & 1, n = r >> 1;
         cp_async16(bS + c * kBChunk + kg * (N * 16) + n * 16, w + (size_t)n * CIN + c * 16 + kg * 8);
     }
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
+    int tile = blockIdx.x;
+    if (tile < tiles) stage(tile, aS);
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    const long long Wf = 2LL * W + 2, Hf = 2LL * H + 2;
+    uint32_t tmem = 0;
+    bool ok = true;
+#pragma unroll 1
+    for (int it = 0; tile < tiles && ok; ++it, tile += gridDim.x) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        // staged, and the previous tile read out of tensor memory
+        __syncthreads();
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem = tmem_base;
+        const uint32_t aT = aS + (uint32_t)((it & 1) * S::kABytes);
+        if (tid == 0) {
 #pragma unroll
-        for (int c = 0; c < CH; ++c) {
+            for (int c = 0; c < CH; ++c) {
 #pragma unroll
-            for (int h = 0; h < N / NMMA; ++h) {
-                const uint64_t ad = umma_desc(aS + c * kAChunk, kConvM * 16, 128);
-                const uint64_t bd = umma_desc(bS + c * kBChunk + h * NMMA * 16, N * 16, 128);
-                const uint32_t accum = c > 0 ? 1u : 0u;
-                asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-                             " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-                             ::"r"(tmem + (uint32_t)(h * NMMA)), "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
-                             : "memory");
+                for (int h = 0; h < N / NMMA; ++h) {
+                    const uint64_t ad = umma_desc(aT + c * kAChunk, kConvM * 16, 128);
+                    const uint64_t bd = umma_desc(bS + c * kBChunk + h * NMMA * 16, N * 16, 128);
+                    const uint32_t accum = c > 0 ? 1u : 0u;
+                    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+                                 " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
+                                 ::"r"(tmem + (uint32_t)(h * NMMA)), "l"(ad), "l"(bd), "r"(idesc), "r"(accum)
+                                 : "memory");
+                }
             }
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                         ::"r"(smem_u32(&mbar)) : "memory");
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-                     ::"r"(smem_u32(&mbar)) : "memory");
-    }
-    // CTA-uniform outcome, so the .sync.aligned TMEM loads never run in a
-    // divergent warp.
-    const bool ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), 0u, err)) != 0;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    if (ok) {
+        // the other buffer's MMAs completed before the last epilogue
+        if (tile + (int)gridDim.x < tiles) stage(tile + gridDim.x, aS + (uint32_t)(((it & 1) ^ 1) * S::kABytes));
+        // CTA-uniform outcome, so the .sync.aligned TMEM loads never run in a
+        // divergent warp.
+        ok = __syncthreads_and(mbar_wait(smem_u32(&mbar), (uint32_t)(it & 1), err)) != 0;
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // warp w owns TMEM lanes 32w..32w+31 = voxels of the tile
-        const long long Pv = P0 + 32 * warp + lane;
-        const int yv = (int)(Pv / Wp), xv = (int)(Pv - (long long)yv * Wp);
+        const int z = tile / tiles_x, Pv = Wp + kConvM * (tile - z * tiles_x) + 32 * warp + lane;
+        const int yv = Pv / Wp, xv = Pv - yv * Wp;
         const bool inside = xv >= 1 && xv <= W && yv >= 1 && yv <= H;
         const int cx = xv - 1, cy = yv - 1;
-        const long long Wf = 2LL * W + 2, Hf = 2LL * H + 2;
 #pragma unroll 1
-        for (int par = 0; par < 8; ++par) {
-            const long long f = ((long long)(2 * z + (par >> 2) + 1) * Hf + (2 * cy + ((par >> 1) & 1) + 1)) * Wf +
-                                (2 * cx + (par & 1) + 1);
+        for (int n2 = 0; n2 < N; n2 += 32) {              // two runs of 16 columns: (parity, 16 channels)
+            uint32_t r[32];
+            const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)n2;
 #pragma unroll
-            for (int n0 = 0; n0 < COUT; n0 += 16) {
-                uint32_t r[16];
-                const uint32_t taddr = tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(par * COUT + n0);
+            for (int h = 0; h < 2; ++h) {
+                uint32_t *q = r + 16 * h;
                 asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                             : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                               "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-                               "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-                             : "r"(taddr) : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (inside) {
-                    __nv_bfloat162 hv[8];
+                             : "=r"(q[0]), "=r"(q[1]), "=r"(q[2]), "=r"(q[3]), "=r"(q[4]), "=r"(q[5]), "=r"(q[6]),
+                               "=r"(q[7]), "=r"(q[8]), "=r"(q[9]), "=r"(q[10]), "=r"(q[11]), "=r"(q[12]),
+                               "=r"(q[13]), "=r"(q[14]), "=r"(q[15])
+                             : "r"(taddr + 16u * h) : "memory");
+            }
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            if (inside) {
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        hv[q] = __floats2bfloat162_rn(__uint_as_float(r[2 * q]) + __ldg(bias + n0 + 2 * q),
-                                                      __uint_as_float(r[2 * q + 1]) + __ldg(bias + n0 + 2 * q + 1));
-                    uint4 *dst = reinterpret_cast<uint4 *>(y + f * ys + n0);
-                    dst[0] = *reinterpret_cast<uint4 *>(&hv[0]);
-                    dst[1] = *reinterpret_cast<uint4 *>(&hv[4]);
+                for (int h = 0; h < 2; ++h) {
+                    const int n = n2 + 16 * h, par = n / COUT, n0 = n % COUT;
+                    const long long f = ((long long)(2 * z + (par >> 2) + 1) * Hf + (2 * cy + ((par >> 1) & 1) + 1)) * Wf +
+                                        (2 * cx + (par & 1) + 1);
+                    uint32_t v[8];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const float4 bq = *reinterpret_cast<const float4 *>(sbias + n0 + 4 * q);
+                        const uint32_t *u = r + 16 * h + 4 * q;
+                        const __nv_bfloat162 lo = __floats2bfloat162_rn(__uint_as_float(u[0]) + bq.x, __uint_as_float(u[1]) + bq.y);
+                        const __nv_bfloat162 hi = __floats2bfloat162_rn(__uint_as_float(u[2]) + bq.z, __uint_as_float(u[3]) + bq.w);
+                        v[2 * q] = *reinterpret_cast<const uint32_t *>(&lo);
+                        v[2 * q + 1] = *reinterpret_cast<const uint32_t *>(&hi);
+                    }
+                    st_bf16x16(y + f * ys + n0, v, wide != 0);
                 }
             }
         }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 0)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kCols) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kCols) : "memory");
 }
 
 template <int CIN, int COUT>
 static cudaError_t launch_up_tc(int W, int H, int D, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
                                 const float *bias, __nv_bfloat16 *y, int ys, int *err, cudaStream_t st) {
-    constexpr int smem = (CIN / 16) * 2 * kConvM * 16 + (CIN / 16) * 2 * (8 * COUT) * 16;
-    cudaError_t e = cudaFuncSetAttribute(k_upconv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    typedef UpShape<CIN, COUT> S;
+    cudaError_t e = cudaFuncSetAttribute(k_upconv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
-    const long long interior = (long long)(W + 2) * H;
-    const dim3 grid((unsigned)((interior + kConvM - 1) / kConvM), (unsigned)D);
-    k_upconv_tc<CIN, COUT><<<grid, 128, smem, st>>>(W, H, D, x, w, bias, y, ys, err);
+    const long long tiles = ((long long)(W + 2) * H + kConvM - 1) / kConvM * D;
+    const long long room = (long long)conv_sm_count() * S::kPerSm;
+    k_upconv_tc<CIN, COUT><<<(unsigned)std::min(tiles, room), 128, S::SMEM, st>>>(W, H, D, x, w, bias, y, ys,
+                                                                                  wide_stores(y, ys, 0), err);
     return cudaGetLastError();
 }
 
