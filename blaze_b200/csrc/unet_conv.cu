@@ -253,40 +253,44 @@ int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 //
 // A tile of 8 x 16 voxels instead of 128 in a row reads 1.4 input voxels per
 // output voxel and plane, not 3, and its block arrives by TMA as one box of 10 x
-// 18 voxels in the canonical K-major layout (core matrices of 8 voxels, 160 bytes
-// from row to row): tap (dy, dx) is the same block seen 160 dy + 16 dx bytes on.
+// 18 voxels of 32 bytes in the K-major layout of the 32-byte swizzle, which is a
+// function of the shared address (slots are whole periods of it), 320 bytes from
+// row to row: tap (dy, dx) is the same block seen 320 dy + 32 dx bytes on.
 //
 // Warps: four read finished accumulators out of TMEM, add bias / ReLU and store;
 // one issues the MMAs (the whole warp runs the loop, so descriptors are uniform
-// values, and one elected lane's instructions take effect); one issues the
-// copies.  They hand over through mbarriers only: full / empty per ring slot,
-// done / free per accumulator.  Every wait is bounded in time; a wait that gives
-// up sets the error flag and ends that warp's loop, which ends the others' at
-// their next wait; before the CTA ends, the MMA warp waits for its last commit
-// and the copy warp for every copy it issued.
+// values, and an elected lane issues); one issues the copies.  They hand over
+// through mbarriers only: full / empty per ring slot, done / free per accumulator.
+// Every wait is bounded in time; a wait that gives up sets the error flag and ends
+// that warp's loop, which ends the others' at their next wait; before the CTA
+// ends, the MMA warp waits for its last commit and the copy warp for every copy
+// it issued.
 //
 // Layers whose weights do not fit (64 or 128 channels in, 64 or 128 out) are cut
 // by output channels: a CTA takes N of them, so the input is staged cout / N
 // times, mostly from L2.
 //
-// Measured (16 -> 16 at 256^3, 32 -> 16 at 256^3, 32 -> 32 at 128^3, 64 -> 32 at
-// 128^3): 461, 786, 139 and 360 us; with an MMA per tap and output plane on 128
-// voxels of a row 738, 1994, 298 and (general kernel) 1146 us.  By parts, 64 ->
-// 64 and 128 -> 64 at 64^3, 64 -> 128 and 128 -> 128 at 32^3: 100, 325, 35 and 96
-// us (general kernel about 228, 456, 62 and 124).  What bounds it
-// now: the copies, whose innermost run is 16 bytes (344 us of the 461 remain
-// without the MMAs and the epilogue), then the MMAs.
+// Measured, us: 16 -> 16 and 32 -> 16 at 256^3 317 and 538, 32 -> 32 and 64 -> 32
+// at 128^3 130 and 290 (an MMA per tap and output plane on 128 voxels of a row: 738,
+// 1994, 298 and, general kernel, 1146); by parts, 64 -> 64 and 128 -> 64 at 64^3
+// 81 and 252 (general kernel about 228 and 456).  What bounds it is the MMA warp: a block
+// costs it about 900 cycles of waits, descriptors and 9 or 10 MMAs, with the
+// copies taken out as with them.  So small layers share an SM, up to four CTAs
+// (16 -> 16: 460 us with two), where the MMAs' operands then take the shared
+// memory's bandwidth (48 cycles an MMA; 44 for 4 KB of voxels and 1.5 KB of
+// weights); the usual case of three planes inside the ring has its own path with
+// constant descriptors, and an elected lane issues (64 -> 32: 360 us without the
+// two).  The swizzle's 32-byte runs against 16-byte ones: 343 against 367 (16 ->
+// 16, before the last two).
 // ---------------------------------------------------------------------------
 constexpr int kZmWorkers = 128;                           // epilogue warps 0-3
 constexpr int kZmThreads = kZmWorkers + 64;               // + the MMA warp + the copy warp
 constexpr int kZmTX = 8, kZmTY = 16;                      // tile (x, y)
-constexpr int kZmRow = (kZmTX + 2) * 16;                  // bytes of one row of a block's half
-constexpr int kZmHalf = (kZmTY + 2) * kZmRow;             // 8 channels of a block
-constexpr int kZmBlock = 2 * kZmHalf;                     // 16 channels of 10 x 18 voxels
-constexpr int kZmSmemOne = 227 * 1024 - 1024;             // dynamic bytes, one CTA per SM
-constexpr int kZmSmemTwo = 228 * 1024 / 2 - 1024 - 512;   // dynamic bytes, two CTAs per SM
+constexpr int kZmRow = (kZmTX + 2) * 32;                  // bytes of one row of a block, 16 channels a voxel
+constexpr int kZmBytes = (kZmTY + 2) * kZmRow;            // a block: 10 x 18 voxels
+constexpr int kZmBlock = (kZmBytes + 1023) / 1024 * 1024; // ring slots, whole periods of the swizzle
+constexpr int zm_room(int ctas) { return ctas == 1 ? 227 * 1024 - 1024 : 228 * 1024 / ctas - 1024 - 512; }   // dynamic bytes a CTA
 constexpr int kZmMaxSlots = 12;
-static_assert(kZmBlock % 128 == 0, "128-byte aligned ring slots");
 
 template <int N, int CIN> struct Zm {
     static constexpr int CH = CIN / 16;
@@ -295,30 +299,38 @@ template <int N, int CIN> struct Zm {
     // at least 3 being read out; a power of two
     static constexpr int R = 2 * (CH - 1) + 6 <= 8 ? 8 : 2 * (CH - 1) + 6 <= 16 ? 16 : 32;
     static constexpr int kCols = R * N;
-    static constexpr bool kTwo = kCols <= 256 && kWeights + 128 + 6 * kZmBlock <= kZmSmemTwo;   // CTAs per SM
-    static constexpr int kRoom = ((kTwo ? kZmSmemTwo : kZmSmemOne) - kWeights - 128) / kZmBlock;
+    // CTAs per SM, as many as tensor memory and shared memory with four ring
+    // slots or more hold
+    static constexpr int slots(int ctas) { return (zm_room(ctas) - kWeights - 1024) / kZmBlock; }
+    static constexpr int kPerSm = kCols * 4 <= 512 && slots(4) >= 4 ? 4 : kCols * 3 <= 512 && slots(3) >= 4 ? 3
+                                  : kCols * 2 <= 512 && slots(2) >= 4 ? 2 : 1;
+    static constexpr int kRoom = slots(kPerSm);
     static constexpr int SL = kRoom < kZmMaxSlots ? kRoom : kZmMaxSlots;
-    static constexpr int kSmem = kWeights + 128 + SL * kZmBlock;
+    static constexpr int kSmem = kWeights + 1024 + SL * kZmBlock;
     static_assert(kCols <= 512 && SL >= 4, "TMEM columns and ring slots");
 };
 
-// One tcgen05.mma, by the lane whose `lead` is set; descriptors as 32-bit halves
-// (offsets only move the address field, in the low half).
-__device__ __forceinline__ void zm_mma(uint32_t lead, uint32_t d, uint32_t a, uint32_t a_hi, uint32_t b, uint32_t b_hi,
-                                       uint32_t idesc, uint32_t acc) {
-    asm volatile("{\n .reg .pred p, q;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n setp.ne.b32 q, %7, 0;\n"
-                 " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
-                 " @q tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n"
-                 ::"r"(d), "r"(a), "r"(a_hi), "r"(b), "r"(b_hi), "r"(idesc), "r"(acc), "r"(lead) : "memory");
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred q;\n elect.sync _|q, 0xffffffff;\n selp.u32 %0, 1, 0, q;\n}\n" : "=r"(p));
+    return p != 0;
 }
-__device__ __forceinline__ void zm_commit(uint32_t lead, uint32_t bar) {
-    asm volatile("{\n .reg .pred q;\n setp.ne.b32 q, %1, 0;\n"
-                 " @q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n}\n"
-                 ::"r"(bar), "r"(lead) : "memory");
+// One tcgen05.mma; descriptors as 32-bit halves (offsets only move the address
+// field, in the low half).
+__device__ __forceinline__ void zm_mma(uint32_t d, uint32_t a, uint32_t a_hi, uint32_t b, uint32_t b_hi,
+                                       uint32_t idesc, uint32_t acc) {
+    asm volatile("{\n .reg .pred p;\n .reg .b64 da, db;\n setp.ne.b32 p, %6, 0;\n"
+                 " mov.b64 da, {%1, %2};\n mov.b64 db, {%3, %4};\n"
+                 " tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n"
+                 ::"r"(d), "r"(a), "r"(a_hi), "r"(b), "r"(b_hi), "r"(idesc), "r"(acc) : "memory");
+}
+__device__ __forceinline__ void zm_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 template <int N, int CIN, bool RELU>
-__global__ void __launch_bounds__(kZmThreads, 1)
+__global__ void __launch_bounds__(kZmThreads, Zm<N, CIN>::kPerSm)
 k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offset,
             const __grid_constant__ CUtensorMap xmap,
             const __nv_bfloat16 *__restrict__ w, const float *__restrict__ bias, __nv_bfloat16 *__restrict__ y,
@@ -329,7 +341,7 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
     constexpr int kTap = 3 * N * 32;                      // bytes of one (chunk, dy, dx)'s weights
     __shared__ __align__(8) uint64_t full[SL], empty[SL], accf[R], acce[R], fin;
     __shared__ uint32_t tmem_base;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int Wp = W + 2, Hp = H + 2;
     const int part = blockIdx.z % parts, cout = parts * N;      // this CTA's output channels: part N .. part N + N - 1
     const int X0 = blockIdx.x * kZmTX, Y0 = blockIdx.y * kZmTY, z0 = (int)(blockIdx.z / parts) * zs;
@@ -352,8 +364,8 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
         init(&fin, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const uint32_t bS = (smem_u32(smem) + 127u) & ~127u;  // weights, then the ring, 128-byte aligned
-    const uint32_t aS = bS + (uint32_t)Z::kWeights;
+    const uint32_t aS = (smem_u32(smem) + 1023u) & ~1023u;     // the ring, then the weights
+    const uint32_t bS = aS + (uint32_t)(SL * kZmBlock);
     // Weights: per (chunk, dy, dx) 3 N rows of 16 channels, K-major: the rows of
     // output plane p - 1 (dz = +1), p (0), p + 1 (-1).
     for (int e = tid; e < 27 * CH * N * 2; e += kZmThreads) {
@@ -433,10 +445,10 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
         // ---- MMA warp ----
         // Every operand address stays below 2^18 bytes, so adding an offset's
         // 16-byte units to the 14-bit address field never carries.
-        const uint64_t a_desc0 = umma_desc(aS, kZmHalf, kZmRow), b_desc0 = umma_desc(bS, 3 * N * 16, 128);
+        const uint64_t a_desc0 = umma_desc(aS, 16, kZmRow) | (uint64_t)6 << 61, b_desc0 = umma_desc(bS, 3 * N * 16, 128);
         const uint32_t a_lo = (uint32_t)a_desc0, a_hi = (uint32_t)(a_desc0 >> 32);
         const uint32_t b_lo = (uint32_t)b_desc0, b_hi = (uint32_t)(b_desc0 >> 32);
-        const uint32_t lead = lane == 0 ? 1u : 0u;
+        const bool lead = elect_one();
         bool ok = true;
         int n = 0, slot = 0;                              // blocks taken; the next one's ring slot
         uint32_t phase = 0;
@@ -464,37 +476,53 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
                 const uint32_t d0 = tmem + (uint32_t)(first * N);
                 auto idesc = [&](int planes) { return umma_idesc_bf16(kConvM, 0) + ((uint32_t)(planes * N / 8) << 17); };
                 auto offset = [&](int planes) { return (uint32_t)(planes * N); };        // weights' rows, 16 bytes each
-                auto tap = [&](int t) { return (uint32_t)(((t / 3) * kZmRow + (t % 3) * 16) >> 4); };
-                int t0 = 0;
-                if (fresh) {                             // tap 0: the new plane overwrites, the others add
-                    const int old = count - 1, h = head < old ? head : old;
-                    if (h > 0) zm_mma(lead, d0, ad0, a_hi, bd0, b_hi, idesc(h), 1u);
-                    if (old > h) zm_mma(lead, tmem, ad0, a_hi, bd0 + offset(h), b_hi, idesc(old - h), 1u);
-                    zm_mma(lead, tmem + (uint32_t)((hi & (R - 1)) * N), ad0, a_hi, bd0 + offset(old), b_hi, idesc(1), 0u);
-                    t0 = 1;
-                }
-                const uint32_t id0 = idesc(head), id1 = idesc(count - head), bd1 = bd0 + offset(head);
-                if (head == count) {
-                    if (t0 == 0) zm_mma(lead, d0, ad0, a_hi, bd0, b_hi, id0, 1u);
+                auto tap = [&](int t) { return (uint32_t)(((t / 3) * kZmRow + (t % 3) * 32) >> 4); };
+                if (lead) {
+                    // tap 0 of a new plane overwrites, the other planes' add
+                    if (hi - lo == 2 && first <= R - 3) {          // three planes, inside the ring
+                        constexpr uint32_t id3 = umma_idesc_bf16(kConvM, 3 * N);
+                        if (fresh) {
+                            zm_mma(d0, ad0, a_hi, bd0, b_hi, umma_idesc_bf16(kConvM, 2 * N), 1u);
+                            zm_mma(d0 + 2 * N, ad0, a_hi, bd0 + offset(2), b_hi, umma_idesc_bf16(kConvM, N), 0u);
+                        } else {
+                            zm_mma(d0, ad0, a_hi, bd0, b_hi, id3, 1u);
+                        }
 #pragma unroll
-                    for (int t = 1; t < 9; ++t)
-                        zm_mma(lead, d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
-                } else {
+                        for (int t = 1; t < 9; ++t)
+                            zm_mma(d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id3, 1u);
+                    } else {
+                        int t0 = 0;
+                        if (fresh) {
+                            const int old = count - 1, h = head < old ? head : old;
+                            if (h > 0) zm_mma(d0, ad0, a_hi, bd0, b_hi, idesc(h), 1u);
+                            if (old > h) zm_mma(tmem, ad0, a_hi, bd0 + offset(h), b_hi, idesc(old - h), 1u);
+                            zm_mma(tmem + (uint32_t)((hi & (R - 1)) * N), ad0, a_hi, bd0 + offset(old), b_hi, idesc(1), 0u);
+                            t0 = 1;
+                        }
+                        const uint32_t id0 = idesc(head), id1 = idesc(count - head), bd1 = bd0 + offset(head);
+                        if (head == count) {
+                            if (t0 == 0) zm_mma(d0, ad0, a_hi, bd0, b_hi, id0, 1u);
+#pragma unroll
+                            for (int t = 1; t < 9; ++t)
+                                zm_mma(d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
+                        } else {
 #pragma unroll 1
-                    for (int t = t0; t < 9; ++t) {
-                        zm_mma(lead, d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
-                        zm_mma(lead, tmem, ad0 + tap(t), a_hi, bd1 + (uint32_t)((t * kTap) >> 4), b_hi, id1, 1u);
+                            for (int t = t0; t < 9; ++t) {
+                                zm_mma(d0, ad0 + tap(t), a_hi, bd0 + (uint32_t)((t * kTap) >> 4), b_hi, id0, 1u);
+                                zm_mma(tmem, ad0 + tap(t), a_hi, bd1 + (uint32_t)((t * kTap) >> 4), b_hi, id1, 1u);
+                            }
+                        }
                     }
+                    zm_commit(smem_u32(&empty[slot]));
+                    if (c == CH - 1 && p - 1 >= z0) zm_commit(smem_u32(&accf[(p - 1 - z0) & (R - 1)]));
                 }
-                zm_commit(lead, smem_u32(&empty[slot]));
-                if (c == CH - 1 && p - 1 >= z0) zm_commit(lead, smem_u32(&accf[(p - 1 - z0) & (R - 1)]));
                 ++n;
                 if (++slot == SL) { slot = 0; phase ^= 1u; }
             }
         // The last MMAs complete before the accumulator columns are released,
         // also when a wait gave up (bounded wait).
         if (n > 0) {
-            zm_commit(lead, smem_u32(&fin));
+            if (lead) zm_commit(smem_u32(&fin));
             mbar_wait(smem_u32(&fin), 0, nullptr);
         }
     } else if (lane == 0) {
@@ -508,11 +536,11 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
                 if (!in_range(p)) continue;
                 if (!mbar_wait(smem_u32(&empty[slot]), phase, err)) { ok = false; break; }
                 const uint32_t bar = smem_u32(&full[slot]);
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kZmBlock) : "memory");
-                asm volatile("cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-                             " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                             ::"r"(aS + (uint32_t)(slot * kZmBlock)), "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(0),
-                               "r"(X0), "r"(Y0), "r"(2 * c), "r"(p + 1), "r"(bar)
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kZmBytes) : "memory");
+                asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                             " [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                             ::"r"(aS + (uint32_t)(slot * kZmBlock)), "l"(reinterpret_cast<uint64_t>(&xmap)), "r"(16 * c),
+                               "r"(X0), "r"(Y0), "r"(p + 1), "r"(bar)
                              : "memory");
                 ++n;
                 if (++slot == SL) { slot = 0; phase ^= 1u; }
@@ -528,21 +556,21 @@ k_conv3d_zm(int W, int H, int D, int zs, int parts, int out_stride, int out_offs
 }
 
 // Tensor map of a padded channels-last activation x (CIN channels, W+2 x
-// H+2 x D+2 voxels from x): dims (8 channels, x, y, 8-channel group, z) with
-// byte strides (2 CIN, row, 16, plane), box (8, 10, 18, 2, 1): one 16-channel
-// chunk of a tile with its border.  The innermost coordinate of every copy is
-// 0, so every copy starts 16-byte aligned; voxels past the tensor read as zeros.
+// H+2 x D+2 voxels from x): dims (channel, x, y, z), box (16, 10, 18, 1): one
+// 16-channel chunk of a tile with its border, 32-byte swizzle.  The innermost
+// coordinate of every copy is a multiple of 16, so every copy starts 32-byte
+// aligned; voxels past the tensor read as zeros.
 static bool zm_tensor_map(CUtensorMap *m, const __nv_bfloat16 *x, const ConvDesc &cd) {
     TensorMapEncodeFn enc = tensor_map_encoder();
     if (!enc || (reinterpret_cast<uintptr_t>(x) & 15) != 0) return false;
     const cuuint64_t Wp = (cuuint64_t)cd.W + 2, Hp = (cuuint64_t)cd.H + 2, Dp = (cuuint64_t)cd.D + 2;
     const cuuint64_t C = (cuuint64_t)cd.cin;
-    const cuuint64_t dims[5] = {8, Wp, Hp, C / 8, Dp};
-    const cuuint64_t strides[4] = {C * 2, Wp * C * 2, 16, Wp * Hp * C * 2};
-    const cuuint32_t box[5] = {8, kZmTX + 2, kZmTY + 2, 2, 1};
-    const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
-    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<__nv_bfloat16 *>(x), dims, strides, box, estr,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+    const cuuint64_t dims[4] = {C, Wp, Hp, Dp};
+    const cuuint64_t strides[3] = {C * 2, Wp * C * 2, Wp * Hp * C * 2};
+    const cuuint32_t box[4] = {16, kZmTX + 2, kZmTY + 2, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<__nv_bfloat16 *>(x), dims, strides, box, estr,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -571,7 +599,7 @@ static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const _
     // zs planes taking zs + 2 + 2 (CH - 1) rounds and about 6 more to start.
     const int parts = cd.cout / N;
     const long long tiles = (long long)((cd.W + kZmTX - 1) / kZmTX) * ((cd.H + kZmTY - 1) / kZmTY) * parts;
-    const long long room = (long long)conv_sm_count() * (Z::kTwo ? 2 : 1);
+    const long long room = (long long)conv_sm_count() * Z::kPerSm;
     int zs = 0;
     long long best = 0;
     for (int v = 4; v <= 64; v <<= 1) {
