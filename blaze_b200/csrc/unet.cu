@@ -77,22 +77,78 @@ struct GridInfo {
     float scale;                          // rho dx^2 / dt
 };
 
-// b, p and r = b - A p of one cell (A p = sum over the in-domain neighbours
-// of p - p_nb, plus p for each p = 0 ghost of a Dirichlet open face), the
-// operator the Gauss-Seidel sweeps solve.
-__device__ __forceinline__ void cell_brp(const GridInfo &g, const CellArr &rhs, const CellArr &p, int i, int j,
-                                         int k, float &b, float &pc, float &r) {
-    pc = p.at(i, j, k, g.W, g.H);
-    b = g.scale * rhs.at(i, j, k, g.W, g.H);
-    float ap = 0.0f;
-    const bool d = g.dirichlet;
-    if (i > 0) ap += pc - p.at(i - 1, j, k, g.W, g.H); else if (d && g.open.xlo) ap += pc;
-    if (i < g.W - 1) ap += pc - p.at(i + 1, j, k, g.W, g.H); else if (d && g.open.xhi) ap += pc;
-    if (j > 0) ap += pc - p.at(i, j - 1, k, g.W, g.H); else if (d && g.open.ylo) ap += pc;
-    if (j < g.H - 1) ap += pc - p.at(i, j + 1, k, g.W, g.H); else if (d && g.open.yhi) ap += pc;
-    if (k > 0) ap += pc - p.at(i, j, k - 1, g.W, g.H); else if (d && g.open.zlo) ap += pc;
-    if (k < g.D - 1) ap += pc - p.at(i, j, k + 1, g.W, g.H); else if (d && g.open.zhi) ap += pc;
-    r = b - ap;
+// One column (i, j) of a field, walked upwards by a warp of 32 neighbouring
+// columns: the z neighbours stay in registers, the x neighbours come from the
+// other lanes, and an element offset moves from plane to plane (in a packed field
+// the two colours swap with it), so a cell costs three loads and no index
+// arithmetic.  Outside the grid every value reads 0.
+struct Column {
+    const float *cur, *oth;              // the colour of the cell, of its neighbours
+    int off, row, plane, left, right;    // of the cell; to its neighbours
+    bool in, xl, xr, yl, yr;             // the column, its neighbours are in the grid
+    float zm, zc, zp;
+    __device__ __forceinline__ Column(const GridInfo &g, const CellArr &a, int i, int j, int k) {
+        in = i >= 0 && i < g.W && j >= 0 && j < g.H;
+        xl = i > 0; xr = i < g.W - 1; yl = j > 0; yr = j < g.H - 1;
+        const bool odd = a.b && ((i + j + k) & 1);
+        cur = odd ? a.b : a.r;
+        oth = a.b && !odd ? a.b : a.r;
+        row = a.b ? g.W >> 1 : g.W;
+        plane = row * g.H;
+        off = (a.b ? i >> 1 : i) + row * j + plane * k;
+        left = a.b ? (i & 1) - 1 : -1;
+        right = a.b ? i & 1 : 1;
+        zm = in && k > 0 && k <= g.D ? __ldg(oth + (off - plane)) : 0.0f;
+        zc = value(g, k);
+        zp = 0.0f;
+    }
+    __device__ __forceinline__ float value(const GridInfo &g, int k) const {
+        return in && k >= 0 && k < g.D ? __ldg(cur + off) : 0.0f;
+    }
+    // A p of the cell at plane k, where the column stands: the sum over the
+    // in-domain neighbours of p - p_nb, plus p for each p = 0 ghost of a Dirichlet
+    // open face (p - 0), nothing at a wall (p - p), the operator the Gauss-Seidel
+    // sweeps solve.  By whole warps.
+    __device__ __forceinline__ float apply(const GridInfo &g, int k) {
+        zp = in && k >= -1 && k < g.D - 1 ? __ldg(oth + (off + plane)) : 0.0f;
+        const float pc = zc;
+        float xm = __shfl_up_sync(0xffffffffu, pc, 1), xp = __shfl_down_sync(0xffffffffu, pc, 1);
+        if (!in || k < 0 || k >= g.D) return 0.0f;
+        const int lane = threadIdx.x & 31;
+        const bool d = g.dirichlet;
+        float ym = d && g.open.ylo ? 0.0f : pc, yp = d && g.open.yhi ? 0.0f : pc;
+        if (lane == 0 && xl) xm = __ldg(oth + (off + left));
+        if (lane == 31 && xr) xp = __ldg(oth + (off + right));
+        if (yl) ym = __ldg(oth + (off - row));
+        if (yr) yp = __ldg(oth + (off + row));
+        if (!xl) xm = d && g.open.xlo ? 0.0f : pc;
+        if (!xr) xp = d && g.open.xhi ? 0.0f : pc;
+        const float zl = k > 0 ? zm : d && g.open.zlo ? 0.0f : pc, zh = k < g.D - 1 ? zp : d && g.open.zhi ? 0.0f : pc;
+        float ap = pc - xm;
+        ap += pc - xp;
+        ap += pc - ym;
+        ap += pc - yp;
+        ap += pc - zl;
+        ap += pc - zh;
+        return ap;
+    }
+    __device__ __forceinline__ void next() {
+        zm = zc;
+        zc = zp;
+        step();
+    }
+    __device__ __forceinline__ void step() {             // for fields only read by value()
+        off += plane;
+        const float *t = cur;
+        cur = oth;
+        oth = t;
+    }
+};
+// Blocks of 32 x 8 columns take kColPlanes planes of them at a time.
+constexpr int kColX = 32, kColY = 8, kColPlanes = 8;
+struct ColTiles { int x, y, z; };
+__host__ __device__ __forceinline__ ColTiles col_tiles(int W, int H, int D) {
+    return {(W + kColX - 1) / kColX, (H + kColY - 1) / kColY, (D + kColPlanes - 1) / kColPlanes};
 }
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -128,19 +184,25 @@ static int one_wave(K kernel) {
     return std::max(1, std::min(kNormBlocks, sms * std::max(1, per)));
 }
 
-// Sums of b^2, p^2, r^2 over the grid (FP64), one triple per block.
-__global__ void __launch_bounds__(kNormThreads)
+// Sums of b^2, p^2, r^2 over the grid (FP64), one triple per block.  Bound
+// by the latency of its loads; five blocks an SM.  256^3 112 us (142 with the 72
+// registers of two planes in flight); with a thread per cell, eight loads and two
+// divisions each, 186.
+__global__ void __launch_bounds__(kNormThreads, 5)
 k_unet_norms(GridInfo g, CellArr rhs, CellArr p, double *partials) {
-    const long long n = (long long)g.W * g.H * g.D;
     double sb = 0.0, sp = 0.0, sr = 0.0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        split3(t, g.W, g.H, i, j, k);
-        float b, pc, r;
-        cell_brp(g, rhs, p, i, j, k, b, pc, r);
-        sb += (double)b * b;
-        sp += (double)pc * pc;
-        sr += (double)r * r;
+    const ColTiles t = col_tiles(g.W, g.H, g.D);
+    for (int q = blockIdx.x; q < t.x * t.y * t.z; q += gridDim.x) {
+        const int i = q % t.x * kColX + (int)(threadIdx.x & 31), j = q / t.x % t.y * kColY + (int)(threadIdx.x >> 5);
+        const int k0 = q / (t.x * t.y) * kColPlanes, k1 = min(k0 + kColPlanes, g.D);
+        Column c(g, p, i, j, k0), cb(g, rhs, i, j, k0);
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k, c.next(), cb.step()) {
+            const float b = g.scale * cb.value(g, k), ap = c.apply(g, k), r = b - ap;
+            sb += (double)b * b;
+            sp += (double)c.zc * c.zc;
+            sr += (double)r * r;
+        }
     }
     __shared__ double s[3][kNormThreads / 32];
     sb = warp_sum_d(sb); sp = warp_sum_d(sp); sr = warp_sum_d(sr);
@@ -188,43 +250,50 @@ __global__ void k_unet_scales(const double *partials, int nblk, double ncells, f
 
 // Input tensor of the crop [o, o + dims) of the grid, halo included: a halo
 // voxel inside the grid carries the grid's values, one outside carries the
-// Neumann-ghost indicator.
-__global__ void k_unet_input(GridInfo g, CellArr rhs, CellArr p, int ox, int oy, int oz, LDims d,
-                             const float *__restrict__ scales, bf16 *__restrict__ x0) {
-    const long long Wp = d.W + 2, Hp = d.H + 2;
-    const long long n = Wp * Hp * (d.D + 2);
-    const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    int xp, yp, zp;
-    split3(t, (int)Wp, (int)Hp, xp, yp, zp);
-    const int i = ox + xp - 1, j = oy + yp - 1, k = oz + zp - 1;
-    float v[kInCh];
+// Neumann-ghost indicator.  Bound by its 32 bytes written per voxel: 256^3 141 us,
+// 4.9 TB/s (a thread per voxel 179).
+__global__ void __launch_bounds__(kColX * kColY)
+k_unet_input(GridInfo g, CellArr rhs, CellArr p, int ox, int oy, int oz, LDims d, const float *__restrict__ scales,
+             bf16 *__restrict__ x0) {
+    const int Wp = d.W + 2, Hp = d.H + 2, Dp = d.D + 2;
+    const int xp = blockIdx.x * kColX + (int)(threadIdx.x & 31), yp = blockIdx.y * kColY + (int)(threadIdx.x >> 5);
+    const int z0 = blockIdx.z * kColPlanes, z1 = min(z0 + kColPlanes, Dp);
+    const int i = ox + xp - 1, j = oy + yp - 1;
+    Column c(g, p, i, j, oz + z0 - 1), cb(g, rhs, i, j, oz + z0 - 1);
+    const float sb = __ldg(scales), sp = __ldg(scales + 1), sr = __ldg(scales + 2);
+#pragma unroll 1
+    for (int zp = z0; zp < z1; ++zp, c.next(), cb.step()) {
+        const int k = oz + zp - 1;
+        const float b = g.scale * cb.value(g, k), ap = c.apply(g, k), r = b - ap;
+        float v[kInCh];
 #pragma unroll
-    for (int c = 0; c < kInCh; ++c) v[c] = 0.0f;
-    if (i >= 0 && i < g.W && j >= 0 && j < g.H && k >= 0 && k < g.D) {
-        float b, pc, r;
-        cell_brp(g, rhs, p, i, j, k, b, pc, r);
-        v[0] = b * scales[0];
-        v[2] = pc * scales[1];
-        v[3] = r * scales[2];
-    } else {
-        // Open in the solve's sense only when it is a p = 0 ghost.
-        const bool d_ = g.dirichlet;
-        bool neumann = false;
-        if (i < 0) neumann |= !(d_ && g.open.xlo);
-        if (i >= g.W) neumann |= !(d_ && g.open.xhi);
-        if (j < 0) neumann |= !(d_ && g.open.ylo);
-        if (j >= g.H) neumann |= !(d_ && g.open.yhi);
-        if (k < 0) neumann |= !(d_ && g.open.zlo);
-        if (k >= g.D) neumann |= !(d_ && g.open.zhi);
-        v[1] = neumann ? 1.0f : 0.0f;
+        for (int q = 0; q < kInCh; ++q) v[q] = 0.0f;
+        if (c.in && k >= 0 && k < g.D) {
+            v[0] = b * sb;
+            v[2] = c.zc * sp;
+            v[3] = r * sr;
+        } else {
+            // Open in the solve's sense only when it is a p = 0 ghost.
+            const bool d_ = g.dirichlet;
+            bool neumann = false;
+            if (i < 0) neumann |= !(d_ && g.open.xlo);
+            if (i >= g.W) neumann |= !(d_ && g.open.xhi);
+            if (j < 0) neumann |= !(d_ && g.open.ylo);
+            if (j >= g.H) neumann |= !(d_ && g.open.yhi);
+            if (k < 0) neumann |= !(d_ && g.open.zlo);
+            if (k >= g.D) neumann |= !(d_ && g.open.zhi);
+            v[1] = neumann ? 1.0f : 0.0f;
+        }
+        if (xp >= Wp || yp >= Hp) continue;
+        __nv_bfloat162 h[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
+        const uint32_t *o = reinterpret_cast<const uint32_t *>(h);
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"        // x0 is 32-byte aligned
+                     ::"l"(x0 + ((long long)xp + (long long)Wp * (yp + (long long)Hp * zp)) * kInCh), "r"(o[0]),
+                       "r"(o[1]), "r"(o[2]), "r"(o[3]), "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7])
+                     : "memory");
     }
-    __nv_bfloat162 h[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) h[q] = __floats2bfloat162_rn(v[2 * q], v[2 * q + 1]);
-    uint4 *dst = reinterpret_cast<uint4 *>(x0 + t * kInCh);
-    dst[0] = *reinterpret_cast<uint4 *>(&h[0]);
-    dst[1] = *reinterpret_cast<uint4 *>(&h[4]);
 }
 
 __device__ __forceinline__ void unpack8(const uint4 &q, float f[8]) {
@@ -345,22 +414,24 @@ __global__ void k_unet_delta(const bf16 *__restrict__ d0b, LDims d, const float 
 }
 
 // Step 3: <r, q>, <q, q>, <d, r> and <d, q> (FP64) with r = b - A p and
-// q = A d, one quadruple per block.
-__global__ void __launch_bounds__(kNormThreads)
+// q = A d, one quadruple per block.  128^3 34 us, with a thread per cell 50.
+__global__ void __launch_bounds__(kNormThreads, 4)
 k_unet_project(GridInfo g, CellArr rhs, CellArr p, CellArr dl, double *partials) {
-    const long long n = (long long)g.W * g.H * g.D;
-    const GridInfo g0{g.W, g.H, g.D, g.open, g.dirichlet, 0.0f};
     double rq = 0.0, qq = 0.0, dr = 0.0, dq = 0.0;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        int i, j, k;
-        split3(t, g.W, g.H, i, j, k);
-        float b, pc, r, zb, dc, mq;
-        cell_brp(g, rhs, p, i, j, k, b, pc, r);
-        cell_brp(g0, rhs, dl, i, j, k, zb, dc, mq);      // with b = 0: mq = -(A d)
-        rq -= (double)r * (double)mq;
-        qq += (double)mq * (double)mq;
-        dr += (double)dc * (double)r;
-        dq -= (double)dc * (double)mq;
+    const ColTiles t = col_tiles(g.W, g.H, g.D);
+    for (int u = blockIdx.x; u < t.x * t.y * t.z; u += gridDim.x) {
+        const int i = u % t.x * kColX + (int)(threadIdx.x & 31), j = u / t.x % t.y * kColY + (int)(threadIdx.x >> 5);
+        const int k0 = u / (t.x * t.y) * kColPlanes, k1 = min(k0 + kColPlanes, g.D);
+        Column c(g, p, i, j, k0), cb(g, rhs, i, j, k0), cd(g, dl, i, j, k0);
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k, c.next(), cd.next(), cb.step()) {
+            const float b = g.scale * cb.value(g, k), ap = c.apply(g, k), r = b - ap;
+            const float mq = 0.0f - cd.apply(g, k);      // -(A d)
+            rq -= (double)r * (double)mq;
+            qq += (double)mq * (double)mq;
+            dr += (double)cd.zc * (double)r;
+            dq -= (double)cd.zc * (double)mq;
+        }
     }
     __shared__ double s[4][kNormThreads / 32];
     double a[4] = {rq, qq, dr, dq};
@@ -754,8 +825,8 @@ int prepare_input(blz_unet *u, const GridInfo &g, const CellArr &rhs, const Cell
     k_unet_norms<<<u->nb_norms, kNormThreads, 0, st>>>(g, rhs, p, u->partials);
     k_unet_scales<<<1, 256, 0, st>>>(u->partials, u->nb_norms, (double)g.W * g.H * g.D, u->kappa, u->scales);
     const LDims &d = u->L[0];
-    const long long n = (long long)(d.W + 2) * (d.H + 2) * (d.D + 2);
-    k_unet_input<<<nblk(n, 256), 256, 0, st>>>(g, rhs, p, org[0], org[1], org[2], d, u->scales, u->X0.base());
+    const ColTiles t = col_tiles(d.W + 2, d.H + 2, d.D + 2);
+    k_unet_input<<<dim3(t.x, t.y, t.z), kColX * kColY, 0, st>>>(g, rhs, p, org[0], org[1], org[2], d, u->scales, u->X0.base());
     u->launches += 3;
     UCKL();
     return BLZ_OK;
