@@ -66,6 +66,10 @@ namespace blz {
 
 constexpr unsigned long long kResWaitNs = 1000ull * 1000ull * 1000ull;   // 1 s; a normal wait takes a microsecond
 
+// Dynamic shared memory a CTA may have.  Every kernel's limit is set to this one
+// value: the limit belongs to the kernel and not to a launch, so a grid's own need
+// would lower it between another thread's setting and launch.
+constexpr int kResSmem = 226 * 1024;
 // Threads a CTA may have: RZ = 2 keeps 32 values of p in registers, RZ = 4
 // keeps 64.
 template <int RZ> constexpr int res_threads() { return RZ == 2 ? 384 : 256; }
@@ -482,7 +486,7 @@ bool shape_of(const Geom &g, int sms, int rz, Shape *out) {
             int TZ = (g.D + nzmax - 1) / nzmax;
             TZ = (TZ + RZ - 1) / RZ * RZ;
             const int threads = Wq * (TY / 2) * (TZ / RZ);
-            if (threads > cap || smem_of(Wq, TY, TZ) > 226 * 1024) continue;
+            if (threads > cap || smem_of(Wq, TY, TZ) > (size_t)kResSmem) continue;
             const int border = res_border(TY, TZ, Wq);
             const int block = std::min(cap, (threads + border + 31) & ~31);
             if (block < threads) continue;
@@ -497,7 +501,7 @@ bool shape_of(const Geom &g, int sms, int rz, Shape *out) {
 
 template <class... P, class... A>
 cudaError_t launch_coop(void (*k)(P...), int ctas, int threads, size_t smem, cudaStream_t st, const A &...args) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1);
