@@ -27,7 +27,7 @@ cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float 
                               SolveCtl *ctl, int chunk, int max_iter, double tol, int variant, cudaStream_t st,
                               cudaGraphExec_t *exec_out, int *body_kernels, int *prologue_kernels, float *q_r,
                               float *q_b, const DefectArrays *dfa, const ResidentWork &res) {
-    cudaError_t err = cudaSuccess;
+    cudaError_t err = cudaSuccess, swept = cudaSuccess;
     cudaGraph_t graph = nullptr, body = nullptr;
     cudaGraphConditionalHandle handle;
     cudaGraphNode_t cond_node;
@@ -66,9 +66,10 @@ cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float 
     CKG(cudaStreamEndCapture(st, &graph));
     // Body: chunk sweeps (timed with the global timer), residual, decision.
     CKG(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    launch_rbgs_sweeps(g, sp, rhs_r, rhs_b, p_r, p_b, chunk, st, &dummy, variant, q_r, q_b, res);
+    swept = launch_rbgs_sweeps(g, sp, rhs_r, rhs_b, p_r, p_b, chunk, st, &dummy, variant, q_r, q_b, res);
     *body_kernels = (int)dummy + check(true);
     CKG(cudaStreamEndCapture(st, &body));
+    CKG(swept);                                          // without its sweeps the loop would only check
     CKG(cudaGraphInstantiate(exec_out, graph, 0));
 done:
     if (err != cudaSuccess) {

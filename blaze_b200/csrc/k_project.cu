@@ -798,13 +798,12 @@ int sweep_variant_count(const Geom &g) {
     return tb_supported(g) ? kSweepVariants : kSegVariants;
 }
 
-void launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r,
-                        const float *rhs_b, float *p_r, float *p_b, int sweeps, cudaStream_t st,
-                        long long *launches, int variant, float *q_r, float *q_b, const ResidentWork &res) {
+cudaError_t launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
+                               float *p_b, int sweeps, cudaStream_t st, long long *launches, int variant, float *q_r,
+                               float *q_b, const ResidentWork &res) {
     if (variant == kResidentVariant && sweeps > 0 && res.work) {
-        launch_resident(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, res, st);   // a launch error stays for cudaGetLastError
         *launches += 1;
-        return;
+        return launch_resident(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, res, st);
     }
     if (variant >= kSegVariants && variant < kSweepVariants && q_r && q_b && tb_supported(g)) {
         // Passes alternate p -> q -> p, an even number of them, so the
@@ -820,7 +819,7 @@ void launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r
         sweeps -= 2 * passes;
         variant = 2;
     }
-    if (sweeps <= 0) return;
+    if (sweeps <= 0) return cudaSuccess;
     if ((g.W & 7) == 0) {
         const int v = (variant >= 0 && variant < kSegVariants) ? variant : 0;
         const int Wq = g.W >> 3, kz = kVariantKZ[v], by = kVariantBY[v];
@@ -849,6 +848,7 @@ void launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r
         }
     }
     *launches += 2LL * sweeps;
+    return cudaSuccess;
 }
 
 // The reference's schedule made race free (FluidSolver.cu:517-599): plane by

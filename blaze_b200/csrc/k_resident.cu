@@ -502,7 +502,6 @@ bool shape_of(const Geom &g, int sms, int rz, Shape *out) {
 template <class... P, class... A>
 cudaError_t launch_coop(void (*k)(P...), int ctas, int threads, size_t smem, cudaStream_t st, const A &...args) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
-    if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1);
     cfg.blockDim = dim3(threads, 1, 1);
@@ -513,7 +512,9 @@ cudaError_t launch_coop(void (*k)(P...), int ctas, int threads, size_t smem, cud
     at[0].val.cooperative = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k, P(args)...);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&cfg, k, P(args)...);
+    if (e != cudaSuccess) cudaGetLastError();            // the caller has it; the next check of a launch must not
+    return e;
 }
 
 bool warp_rows(int Wq, const Shape &s) {

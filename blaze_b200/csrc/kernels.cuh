@@ -101,10 +101,12 @@ bool sweep_variant_uses_tma(int v);
 // Bounded TMA waits of the temporal-blocking pass that gave up since the last
 // call (then reset); nonzero means a pass produced a wrong result.
 unsigned int tb_take_timeouts();
-void launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r,
-                        const float *rhs_b, float *p_r, float *p_b, int sweeps, cudaStream_t st,
-                        long long *launches, int variant = 0, float *q_r = nullptr, float *q_b = nullptr,
-                        const ResidentWork &res = {});
+// Returns whether the on-chip sweeps' launch was taken (a refused one is no node of
+// a capture and leaves the capture valid); the other kernels' launch errors stay
+// for cudaGetLastError.
+cudaError_t launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
+                               float *p_b, int sweeps, cudaStream_t st, long long *launches, int variant = 0,
+                               float *q_r = nullptr, float *q_b = nullptr, const ResidentWork &res = {});
 // The pressure system solved in FP64 (SOR, natural layout) to relative
 // residual tol, the result rounded into p (tight.cu).  Returns 0 or a
 // cudaError_t.

@@ -683,7 +683,7 @@ static int choose_variant(blz_solver *s) {
     // Direct launches first: they set the kernels' attributes outside any
     // capture and warm the SM clock.
     for (int v : cand)
-        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, 4, s->st, &dummy, v, q_r(s), q_b(s), s->res);
+        CK(s, launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, 4, s->st, &dummy, v, q_r(s), q_b(s), s->res));
     CKL(s);
     CK(s, cudaStreamSynchronize(s->st));
     // Each variant is timed as the solve runs it: kTuneSweeps sweeps (one
@@ -703,9 +703,10 @@ static int choose_variant(blz_solver *s) {
         cudaGraph_t gph = nullptr;
         err = cudaStreamBeginCapture(ts, cudaStreamCaptureModeThreadLocal);
         if (err != cudaSuccess) break;
-        launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, kTuneSweeps, ts, &per_graph[v], cand[v], q_r(s),
-                           q_b(s), s->res);
+        const cudaError_t swept = launch_rbgs_sweeps(s->g, sp, s->rhs_r, s->rhs_b, tr, tb, kTuneSweeps, ts, &per_graph[v],
+                                                     cand[v], q_r(s), q_b(s), s->res);
         err = cudaStreamEndCapture(ts, &gph);
+        if (err == cudaSuccess) err = swept;             // an empty graph would be the fastest
         if (err == cudaSuccess) err = cudaGraphInstantiate(&ex[v], gph, 0);
         if (gph) cudaGraphDestroy(gph);
     }
@@ -751,7 +752,7 @@ static int sweeps_on(blz_solver *s, int n, const float *rr, const float *rb, flo
     } else {
         int rc = choose_variant(s);
         if (rc != BLZ_OK) return rc;
-        launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, s->variant, q_r(s), q_b(s), s->res);
+        CK(s, launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, s->variant, q_r(s), q_b(s), s->res));
     }
     CKL(s);
     return BLZ_OK;
@@ -867,11 +868,11 @@ static int warm_start(blz_solver *s, int variant, int *pre) {
             if ((rc = sweeps(s, *pre)) != BLZ_OK) return rc;
             variant = s->variant;
         } else {
-            launch_rbgs_sweeps(s->g, solve_params(P), s->sr_r, s->sr_b, s->sx_r, s->sx_b, *pre, s->st,
-                               &s->launches, variant, q_r(s), q_b(s));
+            CK(s, launch_rbgs_sweeps(s->g, solve_params(P), s->sr_r, s->sr_b, s->sx_r, s->sx_b, *pre, s->st,
+                                     &s->launches, variant, q_r(s), q_b(s)));
         }
-        launch_rbgs_sweeps(s->g, solve_params(P), z_r, z_b, d_r, d_b, *pre, s->st, &s->launches, variant, q_r(s),
-                           q_b(s), s->res);
+        CK(s, launch_rbgs_sweeps(s->g, solve_params(P), z_r, z_b, d_r, d_b, *pre, s->st, &s->launches, variant, q_r(s),
+                                 q_b(s), s->res));
         CKL(s);
     } else {
         *pre = 0;

@@ -2,12 +2,15 @@
 that are refused, the tuner's table, errors that are reported and values that
 are not finite.  Where the sweeps' result matters it is the segment kernel's
 (sweep variant 0), bit for bit."""
+import ctypes as C
+import subprocess
 import threading
 
 import numpy as np
 import pytest
+import torch
 
-from blaze_b200 import FluidSolver, SceneSettings, Timer
+from blaze_b200 import FluidSolver, SceneSettings, Timer, _lib
 from blaze_b200._abi import BLZ_BC_FREE_SURFACE, BLZ_BC_REF_COMPAT
 
 pytestmark = pytest.mark.gpu
@@ -67,3 +70,65 @@ def test_two_threads_sweep_grids_of_different_sizes():
         with make(d, variant=0) as s:
             s.sweeps(calls)
             np.testing.assert_array_equal(p, s.get("P"))
+
+
+class Geom(C.Structure):
+    _fields_ = [("W", C.c_int), ("H", C.c_int), ("D", C.c_int), ("dx", C.c_float), ("dt", C.c_float),
+                ("inv_dx", C.c_float), ("dmin", C.c_float * 3), ("dsize", C.c_float * 3)]
+
+
+class SolveParams(C.Structure):
+    _fields_ = [("scale", C.c_float), ("scale_d", C.c_double), ("open", C.c_bool * 6), ("dirichlet", C.c_int)]
+
+
+class ResidentWork(C.Structure):
+    _fields_ = [("work", C.c_void_p), ("err", C.c_void_p)]
+
+
+def internal(name, restype, argtypes):
+    """A function of the library's own (C++ linkage) by its plain name."""
+    out = subprocess.run(["nm", "-D", "--defined-only", _lib.load()._name], capture_output=True, text=True, check=True).stdout
+    sym = [w[2] for w in map(str.split, out.splitlines()) if f"blz{len(name)}{name}E" in w[2]]
+    assert len(sym) == 1, sym
+    f = getattr(_lib.load(), sym[0])
+    f.restype, f.argtypes = restype, argtypes
+    return f
+
+
+class System:
+    """Device arrays of a small random system and the arguments that describe it."""
+
+    def __init__(self, dims):
+        W, H, D = dims
+        self.g = Geom(W, H, D, 1.0 / W, 1.0 / 24, W, (C.c_float * 3)(), (C.c_float * 3)(1.0, H / W, D / W))
+        self.sp = SolveParams(0.01, 0.01, (C.c_bool * 6)(0, 1, 0, 1, 1, 0), 1)
+        gen = torch.Generator(device="cuda").manual_seed(W + H + D)
+        self.rhs = [torch.randn(W // 2 * H * D, device="cuda", generator=gen) for _ in range(2)]
+        self.p = [torch.randn(W // 2 * H * D, device="cuda", generator=gen) for _ in range(2)]
+        self.bytes = internal("resident_bytes", C.c_size_t, [C.POINTER(Geom)])(C.byref(self.g))
+        self.work = torch.zeros(self.bytes // 4, dtype=torch.int32, device="cuda")
+        self.err = torch.zeros(1, dtype=torch.int32).pin_memory()
+
+    def arrays(self):
+        return [C.c_void_p(t.data_ptr()) for t in self.rhs + self.p]
+
+
+def test_refused_launch_is_an_error_of_the_solve_graph():
+    """A launch of the sweeps that is refused while the solve graph is built
+    (here for want of an error flag) is an error: a graph without sweeps
+    would be kept, and every later solve would only check the residual."""
+    y = System((16, 16, 16))
+    build = internal("build_solve_graph", C.c_int, [C.POINTER(Geom), C.POINTER(SolveParams)] + [C.c_void_p] * 5 +
+                     [C.c_int, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_double, C.c_int] + [C.c_void_p] * 7 +
+                     [C.POINTER(ResidentWork)])
+    partials = torch.zeros(8192, dtype=torch.float64, device="cuda")
+    norm2 = torch.zeros(2, dtype=torch.float64, device="cuda")
+    ctl = torch.zeros(64, dtype=torch.int64, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for err, taken in ((None, False), (y.err.data_ptr(), True)):
+        graph, n = C.c_void_p(), [C.c_int(), C.c_int()]
+        e = build(C.byref(y.g), C.byref(y.sp), *y.arrays(), partials.data_ptr(), 4096, norm2.data_ptr(), ctl.data_ptr(),
+                  10, 20, 1e-3, ON_CHIP, stream.cuda_stream, C.byref(graph), C.byref(n[0]), C.byref(n[1]), None, None,
+                  None, C.byref(ResidentWork(y.work.data_ptr(), err)))
+        assert (e == 0) == taken and bool(graph.value) == taken, (err, e)
