@@ -576,7 +576,8 @@ static float *q_r(blz_solver *s) { return s->scratch + 4 * n_of(s->P, 0); }
 static float *q_b(blz_solver *s) { return s->scratch + 4 * n_of(s->P, 0) + n_of(s->P, 0) / 2; }
 
 static std::mutex g_tune_mu;
-static std::map<std::tuple<int, int, int, int>, int> g_tune_cache;
+// By device, dims, launch shapes offered, on-chip sweeps offered.
+static std::map<std::tuple<int, int, int, int, int, bool>, int> g_tune_cache;
 
 // The tuner's choices persist across processes in a small text file, one
 // line "<device name>|<W>|<H>|<D>|<variants offered>|<variant count> <choice>"
@@ -660,7 +661,7 @@ static int choose_variant(blz_solver *s) {
     std::vector<int> cand;
     if (s->res.work) cand = {0, 4, kResidentVariant};
     else for (int v = 0; v < nv; ++v) cand.push_back(v);
-    const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D * 2 + (nv > kSegVariants ? 1 : 0));
+    const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D, nv, s->res.work != nullptr);
     std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
     {
         std::lock_guard<std::mutex> lk(g_tune_mu);

@@ -132,3 +132,17 @@ def test_refused_launch_is_an_error_of_the_solve_graph():
                   10, 20, 1e-3, ON_CHIP, stream.cuda_stream, C.byref(graph), C.byref(n[0]), C.byref(n[1]), None, None,
                   None, C.byref(ResidentWork(y.work.data_ptr(), err)))
         assert (e == 0) == taken and bool(graph.value) == taken, (err, e)
+
+
+@pytest.mark.parametrize("dims,order", [((392, 16, 16), (0, 1)), ((400, 16, 16), (1, 0))])
+def test_tuner_keeps_solvers_with_other_choices_apart(dims, order, monkeypatch):
+    """Where the two-sweep passes do not apply (W > 384), a solver that may use
+    the on-chip sweeps and one that may not (temporal_block) are offered the
+    same number of launch shapes; each tunes its own choice."""
+    monkeypatch.setenv("BLZ_TUNE_CACHE", "off")
+    monkeypatch.delenv("BLZ_SWEEP_VARIANT", raising=False)
+    for tb in order:
+        with make(dims, variant=-1, temporal_block=tb, maxIterSolve=20) as s:
+            st = s.solve()
+            assert st["sweep_variant"] in ((0, 4, ON_CHIP) if tb == 0 else range(6)), (tb, st)
+            assert s.kernel_launches() > 100, (tb, s.kernel_launches())      # 44 at most without tuning
