@@ -58,7 +58,8 @@ struct blz_solver {
     long long launches = 0;
     blz_unet *warm = nullptr;                   // learned warm start (caller owned)
     int variant = -2;                           // sweep launch shape (-2: not chosen yet)
-    ResidentWork res;                           // on-chip sweeps: exchange buffers, error flag
+    bool on_chip = false;                       // the on-chip sweeps may be chosen
+    ResidentWork res;                           // their exchange buffers (made when first needed) and error flag
     // device-loop solve: instantiated graphs (one per check interval used)
     // and their control block
     struct SolveGraph {
@@ -262,11 +263,10 @@ int blz_create(const blz_params *p, blz_solver **out) {
     ok = ok && cudaMallocHost(&s->h_norm2, 4 * sizeof(double)) == cudaSuccess;   // two norms; the on-chip sweeps' error flag
     ok = ok && cudaMalloc(&s->ctl, sizeof(SolveCtl)) == cudaSuccess;
     ok = ok && cudaMallocHost(&s->h_ctl, sizeof(SolveCtl)) == cudaSuccess;
-    if (ok && p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 && resident_supported(g)) {
-        ok = cudaMalloc(&s->res.work, resident_bytes(g)) == cudaSuccess &&
-             cudaMemset(s->res.work, 0, resident_bytes(g)) == cudaSuccess;
+    if (ok) {
         s->res.err = reinterpret_cast<int *>(s->h_norm2 + 2);
-        if (ok) *s->res.err = 0;
+        *s->res.err = 0;
+        s->on_chip = p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 && resident_supported(g);
     }
     if (!ok) { cudaGetLastError(); int r = fail(s, BLZ_ERR_ALLOC, "device allocation failed for %dx%dx%d", g.W, g.H, g.D); return bail(r); }
     for (auto &ev : s->ev)
@@ -636,6 +636,32 @@ static void tune_file_store(const std::string &key, int v) {
     }
 }
 
+// Makes the on-chip sweeps' exchange buffers (1 MB at 32^3, 13 MB at 128^3) when
+// they are first to run, on a stream of its own: the solver's may be capturing.
+// Where there is no memory for them the solver goes on without.
+static bool prepare_resident(blz_solver *s) {
+    if (s->res.work || !s->on_chip) return s->on_chip;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    const size_t bytes = resident_bytes(s->g);
+    cudaStream_t st = nullptr;
+    void *work = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&work, bytes);
+    if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, bytes, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e == cudaSuccess) {
+        s->res.work = work;
+    } else {
+        cudaGetLastError();
+        cudaFree(work);
+        s->on_chip = false;
+    }
+    if (st) cudaStreamDestroy(st);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    return s->on_chip;
+}
+
 static int choose_variant(blz_solver *s) {
     if (s->variant != -2) return BLZ_OK;
     const int nv = s->P.temporal_block == 1 ? std::min(sweep_variant_count(s->g), kSegVariants)
@@ -646,35 +672,35 @@ static int choose_variant(blz_solver *s) {
         // 20.5), else one cell per thread.
         const char *env = std::getenv("BLZ_SWEEP_VARIANT");
         const int want = s->P.sweep_variant >= 0 ? s->P.sweep_variant : env ? std::atoi(env) : kResidentVariant;
-        s->variant = s->res.work && want == kResidentVariant ? kResidentVariant : -1;
+        s->variant = want == kResidentVariant && prepare_resident(s) ? kResidentVariant : -1;
         return BLZ_OK;
     }
     // A forced choice; the on-chip sweeps (past the launch shapes) only where
     // the grid fits.
-    auto forced = [&](int v) { return v == kResidentVariant && s->res.work ? v : std::max(0, std::min(v, nv - 1)); };
+    auto forced = [&](int v) { return v == kResidentVariant && prepare_resident(s) ? v : std::max(0, std::min(v, nv - 1)); };
     if (s->P.sweep_variant >= 0) { s->variant = forced(s->P.sweep_variant); return BLZ_OK; }
     if (const char *env = std::getenv("BLZ_SWEEP_VARIANT")) { s->variant = forced(std::atoi(env)); return BLZ_OK; }
+    auto key_of = [&] { return std::make_tuple(s->device, s->g.W, s->g.H, s->g.D, nv, s->on_chip); };
+    std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
+    auto known = [&] {                           // the table's or the file's choice, else -1
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tune_cache.find(key_of());
+        if (it != g_tune_cache.end()) return it->second;
+        fkey = tune_key(s->device, s->g, nv, s->on_chip);
+        const int v = tune_file_lookup(fkey);
+        if (!((v >= 0 && v < nv) || (v == kResidentVariant && s->on_chip))) return -1;
+        return g_tune_cache[key_of()] = v;
+    };
+    int v0 = known();
+    if ((v0 < 0 || v0 == kResidentVariant) && s->on_chip && !prepare_resident(s)) v0 = known();   // without the on-chip sweeps
+    if (v0 >= 0) { s->variant = v0; return BLZ_OK; }
     // Candidates: every launch shape, or, for a grid that fits on chip, the on-
     // chip sweeps and the two shapes nearest to them (1.6 to 4.0 us per sweep
     // from 32^3 to 128^3 against 3.8 to 6.7; the temporal-blocking passes take
     // 8 us and more there), so that the first solve of a grid times three.
     std::vector<int> cand;
-    if (s->res.work) cand = {0, 4, kResidentVariant};
+    if (s->on_chip) cand = {0, 4, kResidentVariant};
     else for (int v = 0; v < nv; ++v) cand.push_back(v);
-    const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D, nv, s->res.work != nullptr);
-    std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
-    {
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune_cache.find(key);
-        if (it != g_tune_cache.end()) { s->variant = it->second; return BLZ_OK; }
-        fkey = tune_key(s->device, s->g, nv, s->res.work != nullptr);
-        const int v = tune_file_lookup(fkey);
-        if ((v >= 0 && v < nv) || (v == kResidentVariant && s->res.work)) {
-            g_tune_cache[key] = v;
-            s->variant = v;
-            return BLZ_OK;
-        }
-    }
     const size_t half = n_of(s->P, 0) / 2;
     float *tr = s->scratch, *tb = s->scratch + half;
     CK(s, cudaMemcpyAsync(tr, s->p_r, half * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
@@ -741,7 +767,7 @@ static int choose_variant(blz_solver *s) {
     s->launches += dummy;
     s->variant = best;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key] = best;
+    g_tune_cache[key_of()] = best;
     tune_file_store(fkey, best);
     return BLZ_OK;
 }

@@ -146,3 +146,35 @@ def test_tuner_keeps_solvers_with_other_choices_apart(dims, order, monkeypatch):
             st = s.solve()
             assert st["sweep_variant"] in ((0, 4, ON_CHIP) if tb == 0 else range(6)), (tb, st)
             assert s.kernel_launches() > 100, (tb, s.kernel_launches())      # 44 at most without tuning
+
+
+def test_only_solvers_that_sweep_on_chip_hold_exchange_buffers():
+    """A solver whose sweeps are forced to another kernel takes no more memory
+    than one that may not use the on-chip sweeps (their buffers: 13 MB at
+    128^3)."""
+    def held(**kw):
+        with make((128, 128, 128), **kw) as s:
+            s.sweeps(1)
+            torch.cuda.synchronize()
+            return torch.cuda.mem_get_info()[0]
+
+    held(variant=0)                                       # the allocator's first blocks
+    without, forced = held(variant=0, temporal_block=1), held(variant=0)
+    assert without - forced < 4 << 20, (without, forced)
+
+
+@pytest.mark.parametrize("dims,variant", [((26, 30, 22), -1), ((32, 30, 22), ON_CHIP)])
+def test_first_sweeps_of_a_solver_may_be_captured(dims, variant):
+    """The first call that sweeps on chip, inside a capture of the caller's
+    stream: taken, and each replay runs the sweeps."""
+    with make(dims, variant=variant) as s, make(dims, variant=0) as ref:
+        stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+        _lib.check(_lib.load().blz_set_stream(s._h, C.c_void_p(stream.cuda_stream)), s._h)
+        with torch.cuda.graph(graph, stream=stream):
+            s.sweeps(3)
+        for _ in range(2):
+            graph.replay()
+        torch.cuda.synchronize()
+        ref.sweeps(6)
+        np.testing.assert_array_equal(s.get("P"), ref.get("P"))
+        _lib.check(_lib.load().blz_set_stream(s._h, None), s._h)
