@@ -291,8 +291,8 @@ done:
     return rc;
 }
 
-// Makes the on-chip sweeps' exchange buffers; where there is no memory for them the
-// batch goes on without.
+// Makes the on-chip sweeps' exchange buffers; where there is no memory for them or
+// the context does not take the launches, the batch goes on without.
 static bool prepare_on_chip(blz_batch *b) {
     if (b->res_work || b->waves.empty()) return b->res_work != nullptr;
     cudaError_t e = cudaMalloc(&b->res_work, b->res_bytes);
@@ -301,8 +301,9 @@ static bool prepare_on_chip(blz_batch *b) {
     if (e == cudaSuccess) {
         *b->res_err = 0;
         batch_resident_bind(&b->waves, b->res_work, b->res_err);
-        return true;
+        e = launch_batch_resident(b->waves, b->d_ctl, 0, b->st);
     }
+    if (e == cudaSuccess) return true;
     cudaGetLastError();
     cudaFree(b->res_work);
     b->res_work = nullptr;

@@ -802,8 +802,11 @@ cudaError_t launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float
                                float *p_b, int sweeps, cudaStream_t st, long long *launches, int variant, float *q_r,
                                float *q_b, const ResidentWork &res) {
     if (variant == kResidentVariant && sweeps > 0 && res.work) {
-        *launches += 1;
-        return launch_resident(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, res, st);
+        const cudaError_t e = launch_resident(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, res, st);
+        if (e == cudaSuccess) *launches += 1;
+        // a stream of a context with fewer SMs than when the sweeps were chosen:
+        // the plain kernels below
+        if (e != cudaErrorCooperativeLaunchTooLarge) return e;
     }
     if (variant >= kSegVariants && variant < kSweepVariants && q_r && q_b && tb_supported(g)) {
         // Passes alternate p -> q -> p, an even number of them, so the

@@ -421,6 +421,7 @@ template <int RZ, bool WARPROW, bool RAGGED>
 __global__ void __launch_bounds__(res_threads<RZ>(), 1)
 k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
                 float *p_r, float *p_b, int sweeps, ResParams rs) {
+    if (sweeps <= 0) return;
     res_sweeps<RZ, WARPROW, RAGGED>(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, rs, (int)blockIdx.x);
 }
 
@@ -433,6 +434,7 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
 template <int RZ>
 __global__ void __launch_bounds__(res_threads<RZ>(), 1)
 k_batch_resident(const __grid_constant__ ResidentWave w, const BatchCtl *__restrict__ ctl, int sweeps) {
+    if (sweeps <= 0) return;
     int i = 0;
     while (i + 1 < w.n && (int)blockIdx.x >= w.grid[i + 1].cta0) ++i;
     const ResidentGrid &q = w.grid[i];
@@ -541,7 +543,7 @@ size_t resident_bytes(const Geom &g) {
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st) {
     Shape s;
-    if (!res.work || !res.err || sweeps < 1 || !shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
+    if (!res.work || !res.err || sweeps < 0 || !shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
     const int ctas = s.NY * s.NZ, Wq = quads_of(g);
     const bool ragged = (g.W & 7) != 0;
     ResParams rs{s.NY, s.NZ, s.TY, s.TZ, static_cast<uint4 *>(res.work), nullptr, res.err};

@@ -88,7 +88,9 @@ int  sweep_variant_count(const Geom &g);
 // sweeps (k_resident.cu), for grids that fit (resident_supported).  `work`:
 // resident_bytes(g) bytes of device memory, zeroed once and kept by the caller
 // for launches ordered on one stream; `err`: mapped host memory, set nonzero
-// when a wait between CTAs gave up (the result is then wrong).
+// when a wait between CTAs gave up (the result is then wrong).  A launch without
+// sweeps does nothing but ask whether the context takes it: the CTAs must all run
+// at once, and a context may hold fewer SMs than the device.
 constexpr int kResidentVariant = kSweepVariants;
 struct ResidentWork { void *work = nullptr; int *err = nullptr; };
 bool resident_supported(const Geom &g);
@@ -102,8 +104,9 @@ bool sweep_variant_uses_tma(int v);
 // call (then reset); nonzero means a pass produced a wrong result.
 unsigned int tb_take_timeouts();
 // Returns whether the on-chip sweeps' launch was taken (a refused one is no node of
-// a capture and leaves the capture valid); the other kernels' launch errors stay
-// for cudaGetLastError.
+// a capture and leaves the capture valid; one of too many blocks for the stream's
+// context is replaced by the segment kernel); the other kernels' launch errors
+// stay for cudaGetLastError.
 cudaError_t launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                                float *p_b, int sweeps, cudaStream_t st, long long *launches, int variant = 0,
                                float *q_r = nullptr, float *q_b = nullptr, const ResidentWork &res = {});

@@ -638,7 +638,8 @@ static void tune_file_store(const std::string &key, int v) {
 
 // Makes the on-chip sweeps' exchange buffers (1 MB at 32^3, 13 MB at 128^3) when
 // they are first to run, on a stream of its own: the solver's may be capturing.
-// Where there is no memory for them the solver goes on without.
+// Where there is no memory for them or the context does not take the launch, the
+// solver goes on without.
 static bool prepare_resident(blz_solver *s) {
     if (s->res.work || !s->on_chip) return s->on_chip;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -649,6 +650,8 @@ static bool prepare_resident(blz_solver *s) {
     cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaMalloc(&work, bytes);
     if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, bytes, st);
+    if (e == cudaSuccess)
+        e = launch_resident(s->g, solve_params(s->P), s->rhs_r, s->rhs_b, s->p_r, s->p_b, 0, {work, s->res.err}, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) {
         s->res.work = work;

@@ -3,7 +3,9 @@ that are refused, the tuner's table, errors that are reported and values that
 are not finite.  Where the sweeps' result matters it is the segment kernel's
 (sweep variant 0), bit for bit."""
 import ctypes as C
+import os
 import subprocess
+import sys
 import threading
 
 import numpy as np
@@ -178,3 +180,66 @@ def test_first_sweeps_of_a_solver_may_be_captured(dims, variant):
         ref.sweeps(6)
         np.testing.assert_array_equal(s.get("P"), ref.get("P"))
         _lib.check(_lib.load().blz_set_stream(s._h, None), s._h)
+
+
+_FEW_SMS = r"""
+import sys
+sys.path[:0] = sys.argv[1:3]
+import numpy as np
+from cuda.bindings import driver as cu
+import test_gpu_on_chip_launch as t
+from blaze_b200.batch import Batch
+
+def ok(r):
+    assert r[0] == cu.CUresult.CUDA_SUCCESS, r[0]
+    return r[1] if len(r) == 2 else r[1:]
+
+ok(cu.cuInit(0))
+dev = ok(cu.cuDeviceGet(0))
+sms = ok(cu.cuDeviceGetDevResource(dev, cu.CUdevResourceType.CU_DEV_RESOURCE_TYPE_SM))
+part = ok(cu.cuDevSmResourceSplitByCount(1, sms, 0, 16))[0]
+green = ok(cu.cuGreenCtxCreate(ok(cu.cuDevResourceGenerateDesc(part, 1)), dev,
+                               cu.CUgreenCtxCreate_flags.CU_GREEN_CTX_DEFAULT_STREAM))
+
+# a solver of the whole device, whose stream is then one of the context with few SMs
+with t.make((64, 64, 64)) as s, t.make((64, 64, 64), variant=0) as ref:
+    s.sweeps(3)
+    stream = ok(cu.cuGreenCtxStreamCreate(green, cu.CUstream_flags.CU_STREAM_NON_BLOCKING, 0))
+    t._lib.check(t._lib.load().blz_set_stream(s._h, int(stream)), s._h)
+    s.sweeps(3)
+    ref.sweeps(6)
+    np.testing.assert_array_equal(s.get("P"), ref.get("P"))
+    t._lib.check(t._lib.load().blz_set_stream(s._h, None), s._h)
+
+cu.cuCtxSetCurrent(ok(cu.cuCtxFromGreenCtx(green)))
+
+def solve(dims, variant):
+    with t.make(dims, variant=variant, maxIterSolve=20) as s:
+        st = s.solve()
+        return st["sweep_variant"], s.get("P")
+
+for dims, variant in (((64, 64, 64), -1), ((26, 151, 57), -1), ((64, 64, 64), t.ON_CHIP)):
+    v, p = solve(dims, variant)
+    assert v != t.ON_CHIP, (dims, variant)
+    np.testing.assert_array_equal(p, solve(dims, 0)[1])
+dims = [(64, 64, 64), (48, 40, 36)]
+sims = [t.make(d, variant=0, maxIterSolve=20, tol=1e-9, check_every=10) for d in dims]
+b = Batch(sims)
+assert all(st["sweep_variant"] != t.ON_CHIP for st in b.solve())
+for d, s in zip(dims, sims):
+    np.testing.assert_array_equal(s.get("P"), solve(d, 0)[1])
+b.close()
+print("done")
+"""
+
+
+def test_contexts_with_few_sms_sweep_with_the_other_kernels():
+    """In a context that holds 16 of the SMs, where the blocks of an on-chip launch
+    cannot all run at once and the launch is refused, solvers and batches use the
+    other kernels."""
+    here = os.path.dirname(os.path.abspath(__file__))
+    env = dict(os.environ, BLZ_TUNE_CACHE="off")
+    env.pop("BLZ_SWEEP_VARIANT", None)
+    r = subprocess.run([sys.executable, "-c", _FEW_SMS, os.path.dirname(here), here], env=env, capture_output=True,
+                       text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.endswith("done\n"), r.stderr[-2000:]
