@@ -636,6 +636,19 @@ static void tune_file_store(const std::string &key, int v) {
     }
 }
 
+// The on-chip sweeps flag a bounded wait that gave up (their result is wrong), in
+// host memory.  Sweeps in flight may still set the flag, so it is read by the
+// calls that have waited for the stream, and only by them.
+static bool resident_gave_up(blz_solver *s) {
+    volatile int *flag = s->res.err;
+    if (!*flag) return false;
+    *flag = 0;
+    return true;
+}
+static int take_resident_error(blz_solver *s) {
+    return resident_gave_up(s) ? fail(s, BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up") : BLZ_OK;
+}
+
 // Makes the on-chip sweeps' exchange buffers (1 MB at 32^3, 13 MB at 128^3) when
 // they are first to run, on a stream of its own: the solver's may be capturing.
 // Where there is no memory for them or the context does not take the launch, the
@@ -761,6 +774,11 @@ static int choose_variant(blz_solver *s) {
         if (e) cudaGraphExecDestroy(e);
     cudaStreamDestroy(ts);
     if (err != cudaSuccess) return fail(s, BLZ_ERR_CUDA, "sweep autotuner: %s", cudaGetErrorString(err));
+    // A wait of the on-chip sweeps that gave up while they were timed spoilt the
+    // scratch copies only; it rules them out for this solver, not for the grid.
+    const bool gave_up = resident_gave_up(s);
+    for (int v = 0; v < nc; ++v)
+        if (gave_up && cand[v] == kResidentVariant) t_min[v] = 1e30f;
     const int best = cand[std::min_element(t_min.begin(), t_min.end()) - t_min.begin()];
     if (std::getenv("BLZ_TUNE_VERBOSE")) {
         std::fprintf(stderr, "sweep autotuner %dx%dx%d, us per sweep:", s->g.W, s->g.H, s->g.D);
@@ -769,6 +787,7 @@ static int choose_variant(blz_solver *s) {
     }
     s->launches += dummy;
     s->variant = best;
+    if (gave_up) return BLZ_OK;
     std::lock_guard<std::mutex> lk(g_tune_mu);
     g_tune_cache[key_of()] = best;
     tune_file_store(fkey, best);
@@ -863,18 +882,9 @@ static int solve_device_loop(blz_solver *s, blz_step_stats *st, int chunk) {
 
 static int solve_body(blz_solver *s, blz_step_stats *st);
 
-// The TMA-staged pass counts bounded waits that gave up, the on-chip sweeps flag
-// them; after work that may have used either, they are reported (the result is
-// wrong).  The flag is in host memory: no synchronisation to read it, and a
-// failure of sweeps still in flight shows at the next call that looks.
-static int take_resident_error(blz_solver *s) {
-    if (!s->res.err || !*(volatile int *)s->res.err) return BLZ_OK;
-    *(volatile int *)s->res.err = 0;
-    return fail(s, BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up");
-}
-
+// The TMA-staged pass counts such waits; after work that may have used it they
+// are reported, which waits for the stream.
 static int check_tb_timeouts(blz_solver *s) {
-    if (s->variant == kResidentVariant) return take_resident_error(s);
     if (!sweep_variant_uses_tma(s->variant)) return BLZ_OK;
     CK(s, cudaStreamSynchronize(s->st));
     if (tb_take_timeouts()) return fail(s, BLZ_ERR_TIMEOUT, "temporal-blocking pass: a bounded TMA wait gave up");
@@ -940,6 +950,11 @@ int blz_solve(blz_solver *s, blz_step_stats *st) {
         CK(s, cudaEventRecord(s->ev[9], s->st));
     }
     int rc = solve_body(s, st);
+    if (rc != BLZ_OK && rc != BLZ_ERR_NAN) return rc;
+    if (st || P.tol > 0.0) {                     // the last residual's read waited for the sweeps
+        const int late = take_resident_error(s);
+        if (late != BLZ_OK) return late;
+    }
     if (rc != BLZ_OK) return rc;
     if ((rc = check_tb_timeouts(s)) != BLZ_OK) return rc;
     if (P.defect_correction) {                 // p = RN(p + delta), delta = the exact remainder
@@ -1061,7 +1076,7 @@ int blz_tight_solve(blz_solver *s, double tol, int max_sweeps, double omega, int
     }
     if (sweeps_out) *sweeps_out = sw;
     if (rel_out) *rel_out = rel;
-    return BLZ_OK;
+    return take_resident_error(s);
 }
 
 int blz_gradient(blz_solver *s) {
@@ -1124,7 +1139,8 @@ int blz_step(blz_solver *s, float time, blz_step_stats *st) {
 
 int blz_residual(blz_solver *s, double *res, double *bn) {
     if (!s || !res || !bn) return fail(s, BLZ_ERR_ARG, "null argument");
-    return residual_sync(s, res, bn);
+    const int rc = residual_sync(s, res, bn);
+    return rc != BLZ_OK ? rc : take_resident_error(s);
 }
 
 int blz_perlin(const float *pos3, int n, float scale, int seed, float *out) {
@@ -1191,7 +1207,7 @@ int blz_set_field(blz_solver *s, int f, const float *src, int on_device) {
         CK(s, cudaMemcpyAsync(front_of(s, f), src, n * sizeof(float), kind, s->st));
     }
     CK(s, cudaStreamSynchronize(s->st));
-    return BLZ_OK;
+    return take_resident_error(s);
 }
 
 // ---- z-slab decomposition of the solve ------------------------------------
@@ -1309,5 +1325,7 @@ void solver_batch_view(blz_solver *s, BatchSim *out, const blz_params **P) {
 void solver_flip_front(blz_solver *s) { s->cur ^= 1; }
 void solver_add_launches(blz_solver *s, long long n) { s->launches += n; }
 cudaStream_t solver_stream(blz_solver *s) { return s->st; }
+// The on-chip sweeps' buffers and error flag (tests make a wait run out there).
+ResidentWork *solver_resident(blz_solver *s) { return &s->res; }
 const blz_params *solver_params(blz_solver *s) { return &s->P; }
 } // namespace blz

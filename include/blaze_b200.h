@@ -218,7 +218,17 @@ int  blz_advect(blz_solver *s);                        /* + swap               *
 
 /* Exactly n Gauss-Seidel sweeps (params' order and boundary handling) on the
  * current rhs and p, with no residual checks (the inner loop of
- * gs_solve_kernel, FluidSolver.cu:526-597, run n times).                    */
+ * gs_solve_kernel, FluidSolver.cu:526-597, run n times).
+ *
+ * Sweeps that keep the grid on chip wait for one another's borders inside the
+ * kernel, one second at most.  A wait that gives up (the pressure is then
+ * wrong) is BLZ_ERR_TIMEOUT from the first call that waits for the solver's
+ * stream after it: blz_solve, blz_project or blz_step with statistics or a
+ * tolerance, blz_residual, blz_tight_solve, blz_get_field, blz_set_field, or
+ * the batch's step and solve.  blz_sweeps, and blz_solve, blz_project and
+ * blz_step without statistics and without a tolerance, do not wait and
+ * return BLZ_OK; a caller that reads fields by pointer after them calls one
+ * of the others to learn of it.                                             */
 int  blz_sweeps(blz_solver *s, int n);
 
 /* The current pressure system solved far past the FP32 floor: the iterate

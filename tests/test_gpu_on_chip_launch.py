@@ -11,8 +11,9 @@ import threading
 import numpy as np
 import pytest
 import torch
+from cuda.bindings import runtime as cudart
 
-from blaze_b200 import FluidSolver, SceneSettings, Timer, _lib
+from blaze_b200 import FluidSolver, SceneSettings, Timer, _abi, _lib
 from blaze_b200._abi import BLZ_BC_FREE_SURFACE, BLZ_BC_REF_COMPAT
 
 pytestmark = pytest.mark.gpu
@@ -243,3 +244,58 @@ def test_contexts_with_few_sms_sweep_with_the_other_kernels():
     r = subprocess.run([sys.executable, "-c", _FEW_SMS, os.path.dirname(here), here], env=env, capture_output=True,
                        text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.endswith("done\n"), r.stderr[-2000:]
+
+
+def resident(s):
+    """The solver's exchange buffers and error flag."""
+    return internal("solver_resident", C.POINTER(ResidentWork), [C.c_void_p])(s._h).contents
+
+
+def reports(call):
+    """Whether the call ends with the report of a wait that gave up."""
+    try:
+        call()
+    except _lib.BlazeError as e:
+        assert e.code == _abi.BLZ_ERR_TIMEOUT, e
+        return True
+    return False
+
+
+def test_a_wait_that_gave_up_is_reported_once_by_the_next_call_that_waits():
+    with make((32, 16, 16), maxIterSolve=4) as s:
+        s.sweeps(1)
+        flag = C.cast(resident(s).err, C.POINTER(C.c_int))
+        rhs = s.get("RHS")
+        for call in (lambda: s.get("P"), s.residual, lambda: s.set("RHS", rhs), s.solve, s.project, s.step,
+                     lambda: s.tight_solve(1e-2, 100, 1.5)):
+            flag[0] = 1
+            s.sweeps(1)                                   # does not wait: no report
+            assert reports(call) and not reports(call)
+
+
+def test_a_wait_that_gave_up_while_tuning_rules_the_candidate_out(monkeypatch):
+    monkeypatch.setenv("BLZ_TUNE_CACHE", "off")
+    monkeypatch.delenv("BLZ_SWEEP_VARIANT", raising=False)
+    with make((56, 16, 16), variant=-1, maxIterSolve=4) as s:
+        C.cast(resident(s).err, C.POINTER(C.c_int))[0] = 1
+        assert s.solve()["sweep_variant"] in (0, 4)
+        s.get("P")
+
+
+def test_a_wait_that_runs_out_ends_the_launch():
+    """One block's epoch is set off from the others': its waits and its
+    neighbours' run out, the launch ends, the error is reported, and with the
+    epoch put right the next sweeps are the segment kernel's."""
+    dims = (64, 64, 64)
+    with make(dims) as s, make(dims, variant=0) as ref:
+        s.sweeps(1)
+        p = s.get("P")
+        last = resident(s).work + System(dims).bytes - 4          # the last block's epoch
+        assert cudart.cudaMemset(last, 1, 4)[0] == 0
+        s.sweeps(2)
+        assert reports(lambda: s.get("P"))
+        assert cudart.cudaMemcpy(last, last - 4, 4, cudart.cudaMemcpyKind.cudaMemcpyDeviceToDevice)[0] == 0
+        s.set("P", p)
+        s.sweeps(5)
+        ref.sweeps(6)
+        np.testing.assert_array_equal(s.get("P"), ref.get("P"))
