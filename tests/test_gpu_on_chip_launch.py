@@ -299,3 +299,51 @@ def test_a_wait_that_runs_out_ends_the_launch():
         s.sweeps(5)
         ref.sweeps(6)
         np.testing.assert_array_equal(s.get("P"), ref.get("P"))
+
+
+@pytest.mark.parametrize("dims", [(128, 128, 112), (64, 192, 160), (126, 128, 128), (130, 128, 112)])
+@pytest.mark.parametrize("bc", [BLZ_BC_FREE_SURFACE, BLZ_BC_REF_COMPAT])
+def test_four_planes_per_thread(dims, bc):
+    """Grids near the most that fit: four planes per thread, rows that fill whole
+    warps and rows that are not whole quads."""
+    for batches in ((1,), (2, 5)):
+        out = []
+        for variant in (ON_CHIP, 0):
+            with make(dims, variant=variant, bc=bc) as s:
+                for n in batches:
+                    s.sweeps(n)
+                out.append(s.get("P"))
+        np.testing.assert_array_equal(*out)
+
+
+def test_solves_at_once():
+    """Device-loop solves of three solvers and a batch from four threads, each on its
+    own stream: launches whose blocks must all run at once take turns, and sweep
+    counts and pressures are those of each alone."""
+    from blaze_b200.batch import Batch
+    kw = dict(tol=1e-9, maxIterSolve=400, check_every=20)
+    dims = [(128, 128, 128), (96, 96, 96), (130, 64, 64)]
+    many = [(64, 64, 64), (48, 40, 36), (64, 96, 40)]
+
+    def alone(d):
+        def job():
+            with make(d, **kw) as s:
+                n = [s.solve()["iterations"] for _ in range(4)]
+                return n, s.get("P")
+        return job
+
+    def batched():
+        sims = [make(d, **kw) for d in many]
+        b = Batch(sims)
+        n = [[st["iterations"] for st in b.solve()] for _ in range(4)]
+        out = [(list(k), s.get("P")) for k, s in zip(zip(*n), sims)]
+        b.close()
+        for s in sims:
+            s.close()
+        return out
+
+    got = in_threads([alone(d) for d in dims] + [batched])
+    for d, (n, p) in zip(dims + many, got[:3] + got[3]):
+        with make(d, variant=0, **kw) as s:
+            assert [s.solve()["iterations"] for _ in range(4)] == n, d
+            np.testing.assert_array_equal(s.get("P"), p)
