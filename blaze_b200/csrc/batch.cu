@@ -92,9 +92,8 @@ struct blz_batch {
     int ntiles = 0, tiles_cap = 0;
     size_t tb_smem = 0;                       // largest dynamic shared memory of a tile
     // on-chip sweeps: waves of grids (empty: a grid does not fit), their
-    // exchange buffers (made by the tuner) and error flag
+    // exchange buffers and error flag
     std::vector<ResidentWave> waves;
-    size_t res_bytes = 0;
     void *res_work = nullptr;
     int *res_err = nullptr;
     bool on_chip = false;                     // chosen
@@ -291,26 +290,6 @@ done:
     return rc;
 }
 
-// Makes the on-chip sweeps' exchange buffers; where there is no memory for them or
-// the context does not take the launches, the batch goes on without.
-static bool prepare_on_chip(blz_batch *b) {
-    if (b->res_work || b->waves.empty()) return b->res_work != nullptr;
-    cudaError_t e = cudaMalloc(&b->res_work, b->res_bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(b->res_work, 0, b->res_bytes, b->st);
-    if (e == cudaSuccess && !b->res_err) e = cudaMallocHost(&b->res_err, sizeof(int));
-    if (e == cudaSuccess) {
-        *b->res_err = 0;
-        batch_resident_bind(&b->waves, b->res_work, b->res_err);
-        e = launch_batch_resident(b->waves, b->d_ctl, 0, b->st);
-    }
-    if (e == cudaSuccess) return true;
-    cudaGetLastError();
-    cudaFree(b->res_work);
-    b->res_work = nullptr;
-    b->waves.clear();
-    return false;
-}
-
 // Autotuner: the segment kernel's planes per thread x block size (two sweeps
 // of the whole batch timed) against temporal blocking with 8, 16 or 32
 // planes per tile, scalar or paired-FP32 stencil (four sweeps timed) and, where
@@ -381,7 +360,7 @@ static int tune(blz_batch *b) {
         }
     }
     b->on_chip = false;
-    if (b->force_zc < 0 && e == cudaSuccess && prepare_on_chip(b)) {
+    if (!b->waves.empty() && b->force_zc < 0 && e == cudaSuccess) {
         std::vector<ResidentWave> w = b->waves;
         for (auto &x : w)
             for (int i = 0; i < x.n; ++i) {
@@ -557,7 +536,21 @@ int blz_batch_create(blz_solver *const *sims, int n, blz_batch **out) {
     if (rc == BLZ_OK) ck(cudaMemcpy(b->d_item0, item0.data(), sizeof(long long) * item0.size(), cudaMemcpyHostToDevice), "cudaMemcpy");
     if (rc == BLZ_OK) ck(cudaMemcpy(b->d_blk0, blk0.data(), sizeof(int) * (n + 1), cudaMemcpyHostToDevice), "cudaMemcpy");
     for (int i = 0; i < n && rc == BLZ_OK; ++i) rc = blz_set_stream(sims[i], b->st);
-    if (rc == BLZ_OK && !batch_resident_plan(h.data(), n, &b->waves, &b->res_bytes)) b->waves.clear();
+    size_t res_bytes = 0;
+    if (rc == BLZ_OK && batch_resident_plan(h.data(), n, &b->waves, &res_bytes)) {
+        cudaError_t e = cudaMalloc(&b->res_work, res_bytes);
+        if (e == cudaSuccess) e = cudaMemset(b->res_work, 0, res_bytes);
+        if (e == cudaSuccess) e = cudaMallocHost(&b->res_err, sizeof(int));
+        if (e == cudaSuccess) {
+            *b->res_err = 0;
+            batch_resident_bind(&b->waves, b->res_work, b->res_err);
+        } else {                             // no memory for them: the other kernels
+            cudaGetLastError();
+            cudaFree(b->res_work);
+            b->res_work = nullptr;
+            b->waves.clear();
+        }
+    }
     b->prologue = 1 + 2 + 1;                 // begin, residual + decision, active list
     if (rc != BLZ_OK) {
         release(b);

@@ -421,7 +421,6 @@ template <int RZ, bool WARPROW, bool RAGGED>
 __global__ void __launch_bounds__(res_threads<RZ>(), 1)
 k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const float *__restrict__ rhs_b,
                 float *p_r, float *p_b, int sweeps, ResParams rs) {
-    if (sweeps <= 0) return;
     res_sweeps<RZ, WARPROW, RAGGED>(g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, rs, (int)blockIdx.x);
 }
 
@@ -434,7 +433,6 @@ k_rbgs_resident(Geom g, SolveParams sp, const float *__restrict__ rhs_r, const f
 template <int RZ>
 __global__ void __launch_bounds__(res_threads<RZ>(), 1)
 k_batch_resident(const __grid_constant__ ResidentWave w, const BatchCtl *__restrict__ ctl, int sweeps) {
-    if (sweeps <= 0) return;
     int i = 0;
     while (i + 1 < w.n && (int)blockIdx.x >= w.grid[i + 1].cta0) ++i;
     const ResidentGrid &q = w.grid[i];
@@ -451,6 +449,17 @@ struct Shape { int RZ, NY, NZ, TY, TZ, threads; };
 
 int quads_of(const Geom &g) { return ((g.W >> 1) + 3) >> 2; }      // quads per packed row
 
+// A driver function, null where the driver has none of that name.
+template <class F> F entry_point(const char *name) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return reinterpret_cast<F>(p);
+}
+
 int sm_count() {
     static int cache[64] = {0};
     int dev = 0;
@@ -463,6 +472,20 @@ int sm_count() {
         cache[dev] = coop && n > 0 ? n : -1;
     }
     return cache[dev];
+}
+
+// SMs that the current context holds: a context made for a part of the device's
+// has fewer.
+int context_sms() {
+    static const auto current = entry_point<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
+    static const auto resource =
+        entry_point<CUresult (*)(CUcontext, CUdevResource *, CUdevResourceType)>("cuCtxGetDevResource");
+    CUcontext ctx = nullptr;
+    CUdevResource r = {};
+    if (!current || !resource || current(&ctx) != CUDA_SUCCESS || !ctx ||
+        resource(ctx, &r, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+        return sm_count();
+    return std::min(sm_count(), (int)r.sm.smCount);
 }
 
 size_t smem_of(int Wq, int TY, int TZ) {
@@ -527,7 +550,7 @@ bool warp_rows(int Wq, const Shape &s) {
 
 bool resident_supported(const Geom &g) {
     Shape s;
-    return shape_of(g, sm_count(), 0, &s);
+    return shape_of(g, sm_count(), 0, &s) && s.NY * s.NZ <= context_sms();
 }
 
 static size_t halo_quads(const Geom &g, const Shape &s) {
@@ -543,7 +566,7 @@ size_t resident_bytes(const Geom &g) {
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st) {
     Shape s;
-    if (!res.work || !res.err || sweeps < 0 || !shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
+    if (!res.work || !res.err || sweeps < 1 || !shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
     const int ctas = s.NY * s.NZ, Wq = quads_of(g);
     const bool ragged = (g.W & 7) != 0;
     ResParams rs{s.NY, s.NZ, s.TY, s.TZ, static_cast<uint4 *>(res.work), nullptr, res.err};
@@ -564,7 +587,7 @@ cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *r
 // most cells per CTA.  Two planes per thread where that takes no more waves than
 // four.  False where a grid does not fit.
 bool batch_resident_plan(const BatchSim *sims, int n, std::vector<ResidentWave> *waves, size_t *bytes) {
-    const int sms = sm_count();
+    const int sms = context_sms();
     struct Item { int sim, ctas; Shape s; };
     auto work_of = [&](const Item &x) { return (long long)quads_of(sims[x.sim].g) * (x.s.TY * x.s.TZ + x.s.TY + x.s.TZ); };
     std::vector<std::vector<Item>> best;

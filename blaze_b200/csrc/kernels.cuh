@@ -88,9 +88,8 @@ int  sweep_variant_count(const Geom &g);
 // sweeps (k_resident.cu), for grids that fit (resident_supported).  `work`:
 // resident_bytes(g) bytes of device memory, zeroed once and kept by the caller
 // for launches ordered on one stream; `err`: mapped host memory, set nonzero
-// when a wait between CTAs gave up (the result is then wrong).  A launch without
-// sweeps does nothing but ask whether the context takes it: the CTAs must all run
-// at once, and a context may hold fewer SMs than the device.
+// when a wait between CTAs gave up (the result is then wrong).  The CTAs must all
+// run at once: resident_supported also asks how many SMs the current context holds.
 constexpr int kResidentVariant = kSweepVariants;
 struct ResidentWork { void *work = nullptr; int *err = nullptr; };
 bool resident_supported(const Geom &g);

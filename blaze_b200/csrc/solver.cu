@@ -58,8 +58,7 @@ struct blz_solver {
     long long launches = 0;
     blz_unet *warm = nullptr;                   // learned warm start (caller owned)
     int variant = -2;                           // sweep launch shape (-2: not chosen yet)
-    bool on_chip = false;                       // the on-chip sweeps may be chosen
-    ResidentWork res;                           // their exchange buffers (made when first needed) and error flag
+    ResidentWork res;                           // on-chip sweeps: exchange buffers (behind scratch; null: never chosen), error flag
     // device-loop solve: instantiated graphs (one per check interval used)
     // and their control block
     struct SolveGraph {
@@ -187,7 +186,6 @@ static void release(blz_solver *s) {
     for (auto &gr : s->graphs)
         if (gr.exec) cudaGraphExecDestroy(gr.exec);
     cudaFree(s->ctl);
-    cudaFree(s->res.work);
     if (s->h_ctl) cudaFreeHost(s->h_ctl);
     for (auto &e : s->ev) if (e) cudaEventDestroy(e);
     if (s->own_stream && s->st) cudaStreamDestroy(s->st);
@@ -244,7 +242,18 @@ int blz_create(const blz_params *p, blz_solver **out) {
     } else {
         s->sr_r = s->rhs_r; s->sr_b = s->rhs_b; s->sx_r = s->p_r; s->sx_b = s->p_b;
     }
-    ok = ok && alloc(&s->scratch, 6 * nT);
+    // The on-chip sweeps' exchange buffers (0.9 MB at 32^3, 13.5 MB at 128^3) lie
+    // behind the scratch arrays: an allocation of their own takes longer than all
+    // else they need.  A solver that has no memory for them does without.
+    const size_t work_at = (6 * nT + 63) / 64 * 64;
+    const bool on_chip = p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 &&
+                         (p->sweep_variant < 0 || p->sweep_variant == kResidentVariant) && resident_supported(g);
+    if (ok && on_chip && alloc(&s->scratch, work_at + resident_bytes(g) / sizeof(float))) {
+        s->res.work = s->scratch + work_at;
+    } else if (ok) {
+        if (on_chip) cudaGetLastError();
+        ok = alloc(&s->scratch, 6 * nT);
+    }
     if (p->density_field) ok = ok && alloc(&s->Dn[0], nT) && alloc(&s->Dn[1], nT);
     (void)nU; (void)nV; (void)nW;
     s->cap_parts = std::max(p->max_particles, 1);
@@ -266,7 +275,6 @@ int blz_create(const blz_params *p, blz_solver **out) {
     if (ok) {
         s->res.err = reinterpret_cast<int *>(s->h_norm2 + 2);
         *s->res.err = 0;
-        s->on_chip = p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 && resident_supported(g);
     }
     if (!ok) { cudaGetLastError(); int r = fail(s, BLZ_ERR_ALLOC, "device allocation failed for %dx%dx%d", g.W, g.H, g.D); return bail(r); }
     for (auto &ev : s->ev)
@@ -649,35 +657,6 @@ static int take_resident_error(blz_solver *s) {
     return resident_gave_up(s) ? fail(s, BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up") : BLZ_OK;
 }
 
-// Makes the on-chip sweeps' exchange buffers (1 MB at 32^3, 13 MB at 128^3) when
-// they are first to run, on a stream of its own: the solver's may be capturing.
-// Where there is no memory for them or the context does not take the launch, the
-// solver goes on without.
-static bool prepare_resident(blz_solver *s) {
-    if (s->res.work || !s->on_chip) return s->on_chip;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    const size_t bytes = resident_bytes(s->g);
-    cudaStream_t st = nullptr;
-    void *work = nullptr;
-    cudaError_t e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
-    if (e == cudaSuccess) e = cudaMalloc(&work, bytes);
-    if (e == cudaSuccess) e = cudaMemsetAsync(work, 0, bytes, st);
-    if (e == cudaSuccess)
-        e = launch_resident(s->g, solve_params(s->P), s->rhs_r, s->rhs_b, s->p_r, s->p_b, 0, {work, s->res.err}, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e == cudaSuccess) {
-        s->res.work = work;
-    } else {
-        cudaGetLastError();
-        cudaFree(work);
-        s->on_chip = false;
-    }
-    if (st) cudaStreamDestroy(st);
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    return s->on_chip;
-}
-
 static int choose_variant(blz_solver *s) {
     if (s->variant != -2) return BLZ_OK;
     const int nv = s->P.temporal_block == 1 ? std::min(sweep_variant_count(s->g), kSegVariants)
@@ -688,35 +667,35 @@ static int choose_variant(blz_solver *s) {
         // 20.5), else one cell per thread.
         const char *env = std::getenv("BLZ_SWEEP_VARIANT");
         const int want = s->P.sweep_variant >= 0 ? s->P.sweep_variant : env ? std::atoi(env) : kResidentVariant;
-        s->variant = want == kResidentVariant && prepare_resident(s) ? kResidentVariant : -1;
+        s->variant = s->res.work && want == kResidentVariant ? kResidentVariant : -1;
         return BLZ_OK;
     }
     // A forced choice; the on-chip sweeps (past the launch shapes) only where
     // the grid fits.
-    auto forced = [&](int v) { return v == kResidentVariant && prepare_resident(s) ? v : std::max(0, std::min(v, nv - 1)); };
+    auto forced = [&](int v) { return v == kResidentVariant && s->res.work ? v : std::max(0, std::min(v, nv - 1)); };
     if (s->P.sweep_variant >= 0) { s->variant = forced(s->P.sweep_variant); return BLZ_OK; }
     if (const char *env = std::getenv("BLZ_SWEEP_VARIANT")) { s->variant = forced(std::atoi(env)); return BLZ_OK; }
-    auto key_of = [&] { return std::make_tuple(s->device, s->g.W, s->g.H, s->g.D, nv, s->on_chip); };
-    std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
-    auto known = [&] {                           // the table's or the file's choice, else -1
-        std::lock_guard<std::mutex> lk(g_tune_mu);
-        auto it = g_tune_cache.find(key_of());
-        if (it != g_tune_cache.end()) return it->second;
-        fkey = tune_key(s->device, s->g, nv, s->on_chip);
-        const int v = tune_file_lookup(fkey);
-        if (!((v >= 0 && v < nv) || (v == kResidentVariant && s->on_chip))) return -1;
-        return g_tune_cache[key_of()] = v;
-    };
-    int v0 = known();
-    if ((v0 < 0 || v0 == kResidentVariant) && s->on_chip && !prepare_resident(s)) v0 = known();   // without the on-chip sweeps
-    if (v0 >= 0) { s->variant = v0; return BLZ_OK; }
     // Candidates: every launch shape, or, for a grid that fits on chip, the on-
     // chip sweeps and the two shapes nearest to them (1.6 to 4.0 us per sweep
     // from 32^3 to 128^3 against 3.8 to 6.7; the temporal-blocking passes take
     // 8 us and more there), so that the first solve of a grid times three.
     std::vector<int> cand;
-    if (s->on_chip) cand = {0, 4, kResidentVariant};
+    if (s->res.work) cand = {0, 4, kResidentVariant};
     else for (int v = 0; v < nv; ++v) cand.push_back(v);
+    const auto key = std::make_tuple(s->device, s->g.W, s->g.H, s->g.D, nv, s->res.work != nullptr);
+    std::string fkey;                            // formed only for a grid this process has not met: it asks for the device's properties
+    {
+        std::lock_guard<std::mutex> lk(g_tune_mu);
+        auto it = g_tune_cache.find(key);
+        if (it != g_tune_cache.end()) { s->variant = it->second; return BLZ_OK; }
+        fkey = tune_key(s->device, s->g, nv, s->res.work != nullptr);
+        const int v = tune_file_lookup(fkey);
+        if ((v >= 0 && v < nv) || (v == kResidentVariant && s->res.work)) {
+            g_tune_cache[key] = v;
+            s->variant = v;
+            return BLZ_OK;
+        }
+    }
     const size_t half = n_of(s->P, 0) / 2;
     float *tr = s->scratch, *tb = s->scratch + half;
     CK(s, cudaMemcpyAsync(tr, s->p_r, half * sizeof(float), cudaMemcpyDeviceToDevice, s->st));
@@ -789,7 +768,7 @@ static int choose_variant(blz_solver *s) {
     s->variant = best;
     if (gave_up) return BLZ_OK;
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    g_tune_cache[key_of()] = best;
+    g_tune_cache[key] = best;
     tune_file_store(fkey, best);
     return BLZ_OK;
 }

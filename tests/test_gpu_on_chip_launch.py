@@ -226,7 +226,7 @@ for dims, variant in (((64, 64, 64), -1), ((26, 151, 57), -1), ((64, 64, 64), t.
 dims = [(64, 64, 64), (48, 40, 36)]
 sims = [t.make(d, variant=0, maxIterSolve=20, tol=1e-9, check_every=10) for d in dims]
 b = Batch(sims)
-assert all(st["sweep_variant"] != t.ON_CHIP for st in b.solve())
+b.solve()                                                # small grids may still fit the SMs there are
 for d, s in zip(dims, sims):
     np.testing.assert_array_equal(s.get("P"), solve(d, 0)[1])
 b.close()
@@ -236,8 +236,8 @@ print("done")
 
 def test_contexts_with_few_sms_sweep_with_the_other_kernels():
     """In a context that holds 16 of the SMs, where the blocks of an on-chip launch
-    cannot all run at once and the launch is refused, solvers and batches use the
-    other kernels."""
+    cannot all run at once, solvers use the other kernels, and batches either
+    those or a plan for 16 SMs."""
     here = os.path.dirname(os.path.abspath(__file__))
     env = dict(os.environ, BLZ_TUNE_CACHE="off")
     env.pop("BLZ_SWEEP_VARIANT", None)
