@@ -202,6 +202,7 @@ static int build_graph(blz_batch *b, bool with_stages, cudaGraphExec_t *out, lon
     cudaGraphConditionalHandle h;
     cudaGraphNode_t cond;
     int rc = BLZ_OK;
+    bool broken = false;                      // the body's capture has not ended well
     long long l0 = 0, l1 = 0;
     auto launches_now = [&]() {
         long long t = 0;
@@ -259,6 +260,7 @@ static int build_graph(blz_batch *b, bool with_stages, cudaGraphExec_t *out, lon
         const cudaError_t launched = capture_body(b, h);
         cudaGraph_t g2 = nullptr;
         e = cudaStreamEndCapture(b->st, &g2);
+        broken = e != cudaSuccess;
         if (e == cudaSuccess) e = launched;
     }
     if (e != cudaSuccess) goto done;
@@ -286,7 +288,9 @@ done:
         cudaGetLastError();
         if (rc == BLZ_OK) rc = bfail(BLZ_ERR_CUDA, "building the batch graph failed: %s", cudaGetErrorString(e));
     }
-    if (graph) cudaGraphDestroy(graph);
+    // A graph whose body's capture failed is left: destroying it crashes the driver
+    // (580.159).
+    if (graph && !broken) cudaGraphDestroy(graph);
     return rc;
 }
 
@@ -541,9 +545,9 @@ int blz_batch_create(blz_solver *const *sims, int n, blz_batch **out) {
         cudaError_t e = cudaMalloc(&b->res_work, res_bytes);
         if (e == cudaSuccess) e = cudaMemset(b->res_work, 0, res_bytes);
         if (e == cudaSuccess) e = cudaMallocHost(&b->res_err, sizeof(int));
+        if (e == cudaSuccess) e = batch_resident_bind(&b->waves, b->res_work, b->res_err);
         if (e == cudaSuccess) {
             *b->res_err = 0;
-            batch_resident_bind(&b->waves, b->res_work, b->res_err);
         } else {                             // no memory for them: the other kernels
             cudaGetLastError();
             cudaFree(b->res_work);

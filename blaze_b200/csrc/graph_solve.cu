@@ -32,6 +32,7 @@ cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float 
     cudaGraphConditionalHandle handle;
     cudaGraphNode_t cond_node;
     long long dummy = 0;
+    bool broken = false;                                 // the body's capture has not ended well
     *exec_out = nullptr;
     // The stopping test: the FP64 residual of (rhs, p); for a defect-
     // correction solve (after sweeps) d folded into p and a fresh defect,
@@ -66,9 +67,11 @@ cudaError_t build_solve_graph(const Geom &g, const SolveParams &sp, const float 
     CKG(cudaStreamEndCapture(st, &graph));
     // Body: chunk sweeps (timed with the global timer), residual, decision.
     CKG(cudaStreamBeginCaptureToGraph(st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+    broken = true;
     swept = launch_rbgs_sweeps(g, sp, rhs_r, rhs_b, p_r, p_b, chunk, st, &dummy, variant, q_r, q_b, res);
     *body_kernels = (int)dummy + check(true);
     CKG(cudaStreamEndCapture(st, &body));
+    broken = false;
     CKG(swept);                                          // without its sweeps the loop would only check
     CKG(cudaGraphInstantiate(exec_out, graph, 0));
 done:
@@ -81,7 +84,9 @@ done:
         }
         cudaGetLastError();
     }
-    if (graph) cudaGraphDestroy(graph);
+    // A graph whose body's capture failed is left: destroying it crashes the driver
+    // (580.159).
+    if (graph && !broken) cudaGraphDestroy(graph);
     return err;
 }
 

@@ -378,20 +378,41 @@ __global__ void __launch_bounds__(256) k_advect(Geom g, AdvectArrays a) {
 // cell, where k_advect takes 0.16 at 96^3.
 constexpr int kTileGrids = 888;
 
+constexpr int tile_smem(bool dens) { return (dens ? 5 : 4) * kTileNodes * (int)sizeof(float); }
+
+template <int SCHEME>
+static cudaError_t prepare_scheme(bool dens) {
+    return dens ? allow_smem((const void *)k_advect_tile<SCHEME, true>, tile_smem(true))
+                : allow_smem((const void *)k_advect_tile<SCHEME, false>, tile_smem(false));
+}
+
+static bool wide(const Geom &g) { return g.W >= (1 << 23) - 1 || g.H >= (1 << 23) - 1 || g.D >= (1 << 23) - 1; }
+static dim3 tiles(const Geom &g) { return dim3((g.W + kTX - 1) / kTX, (g.H + kTY - 1) / kTY, (g.D + kTZ - 1) / kTZ); }
+static bool tiled(const Geom &g) {
+    const dim3 t = tiles(g);
+    return !wide(g) && (int)(t.x * t.y * t.z) >= kTileGrids;
+}
+
+cudaError_t advect_prepare(const Geom &g, int scheme, bool dens) {
+    if (!tiled(g)) return cudaSuccess;
+    return scheme == BLZ_ADVECT_EULER ? prepare_scheme<BLZ_ADVECT_EULER>(dens)
+           : scheme == BLZ_ADVECT_RK2 ? prepare_scheme<BLZ_ADVECT_RK2>(dens) : prepare_scheme<BLZ_ADVECT_RK3>(dens);
+}
+
 template <int SCHEME, bool DENS>
 static void launch_scheme(const Geom &g, const AdvectArrays &a, cudaStream_t st) {
-    const bool wide = g.W >= (1 << 23) - 1 || g.H >= (1 << 23) - 1 || g.D >= (1 << 23) - 1;
-    const int nx = (g.W + kTX - 1) / kTX, ny = (g.H + kTY - 1) / kTY, nz = (g.D + kTZ - 1) / kTZ, n = nx * ny * nz;
-    if (wide || n < kTileGrids) {
-        if (wide) k_advect<SCHEME, DENS, true><<<face_grid(g), face_block(), 0, st>>>(g, a);
+    if (!tiled(g)) {
+        if (wide(g)) k_advect<SCHEME, DENS, true><<<face_grid(g), face_block(), 0, st>>>(g, a);
         else k_advect<SCHEME, DENS, false><<<face_grid(g), face_block(), 0, st>>>(g, a);
         return;
     }
-    constexpr int smem = (DENS ? 5 : 4) * kTileNodes * (int)sizeof(float);
-    cudaFuncSetAttribute(k_advect_tile<SCHEME, DENS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    constexpr int smem = tile_smem(DENS);
+    allow_smem((const void *)k_advect_tile<SCHEME, DENS>, smem);
+    const dim3 t = tiles(g);
+    const int n = (int)(t.x * t.y * t.z);
     const long long last = (long long)g.H * g.D + (long long)g.W * g.D + (long long)g.W * g.H;
     k_advect_tile<SCHEME, DENS><<<n + (unsigned)((last + kAdvThreads - 1) / kAdvThreads), kAdvThreads, smem, st>>>(
-        g, a, nx, ny, n);
+        g, a, (int)t.x, (int)t.y, n);
 }
 
 void launch_advect(const Geom &g, const float *T, const float *U, const float *V, const float *W,

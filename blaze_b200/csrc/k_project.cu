@@ -7,7 +7,10 @@
 // all rows contiguous; red cells of a row are even or odd i according to the
 // row parity (j+k)&1.
 #include <algorithm>
+#include <mutex>
+#include <set>
 #include <type_traits>
+#include <utility>
 
 #include <cuda.h>   // CUtensorMap and its enums; the encoder comes from cudaGetDriverEntryPoint
 
@@ -621,6 +624,20 @@ static size_t tb_smem(const Geom &g, int TY) {
 static size_t tb_smem_tma(const Geom &g, int TY) {
     const int Wq = g.W >> 3, ra = tb_rows_alloc(TY);
     return 128 + (size_t)kTbDenseSlots * tb_dense_slot_bytes(Wq, ra) + sizeof(float4) * 8 * (size_t)ra * (Wq + 1);
+}
+
+cudaError_t allow_smem(const void *kernel, int bytes) {
+    static const auto context_id = driver_function<CUresult (*)(CUcontext, unsigned long long *)>("cuCtxGetId");
+    static std::mutex m;
+    static std::set<std::pair<const void *, unsigned long long>> done;
+    unsigned long long id = 0;                           // of the current context; ids are not used again
+    if (!context_id || context_id(nullptr, &id) != CUDA_SUCCESS)
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    std::lock_guard<std::mutex> lk(m);
+    if (done.count({kernel, id})) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) done.insert({kernel, id});
+    return e;
 }
 
 TensorMapEncodeFn tensor_map_encoder() {

@@ -67,8 +67,8 @@ namespace blz {
 constexpr unsigned long long kResWaitNs = 1000ull * 1000ull * 1000ull;   // 1 s; a normal wait takes a microsecond
 
 // Dynamic shared memory a CTA may have.  Every kernel's limit is set to this one
-// value: the limit belongs to the kernel and not to a launch, so a grid's own need
-// would lower it between another thread's setting and launch.
+// value, once: the limit belongs to the kernel and not to a launch, so a grid's own
+// need would lower it between another thread's setting and launch.
 constexpr int kResSmem = 226 * 1024;
 // Threads a CTA may have: RZ = 2 keeps 32 values of p in registers, RZ = 4
 // keeps 64.
@@ -449,17 +449,6 @@ struct Shape { int RZ, NY, NZ, TY, TZ, threads; };
 
 int quads_of(const Geom &g) { return ((g.W >> 1) + 3) >> 2; }      // quads per packed row
 
-// A driver function, null where the driver has none of that name.
-template <class F> F entry_point(const char *name) {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
-        cudaGetLastError();
-        return nullptr;
-    }
-    return reinterpret_cast<F>(p);
-}
-
 int sm_count() {
     static int cache[64] = {0};
     int dev = 0;
@@ -477,9 +466,9 @@ int sm_count() {
 // SMs that the current context holds: a context made for a part of the device's
 // has fewer.
 int context_sms() {
-    static const auto current = entry_point<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
+    static const auto current = driver_function<CUresult (*)(CUcontext *)>("cuCtxGetCurrent");
     static const auto resource =
-        entry_point<CUresult (*)(CUcontext, CUdevResource *, CUdevResourceType)>("cuCtxGetDevResource");
+        driver_function<CUresult (*)(CUcontext, CUdevResource *, CUdevResourceType)>("cuCtxGetDevResource");
     CUcontext ctx = nullptr;
     CUdevResource r = {};
     if (!current || !resource || current(&ctx) != CUDA_SUCCESS || !ctx ||
@@ -526,7 +515,7 @@ bool shape_of(const Geom &g, int sms, int rz, Shape *out) {
 
 template <class... P, class... A>
 cudaError_t launch_coop(void (*k)(P...), int ctas, int threads, size_t smem, cudaStream_t st, const A &...args) {
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kResSmem);
+    cudaError_t e = allow_smem((const void *)k, kResSmem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(ctas, 1, 1);
     cfg.blockDim = dim3(threads, 1, 1);
@@ -563,22 +552,29 @@ size_t resident_bytes(const Geom &g) {
     return halo_quads(g, s) * sizeof(uint4) + (size_t)s.NY * s.NZ * sizeof(unsigned);
 }
 
+typedef void (*ResidentKernel)(Geom, SolveParams, const float *, const float *, float *, float *, int, ResParams);
+static ResidentKernel resident_kernel(const Geom &g, const Shape &s) {
+    const bool ragged = (g.W & 7) != 0, warprow = warp_rows(quads_of(g), s);
+    if (s.RZ == 2)
+        return ragged ? k_rbgs_resident<2, false, true> : warprow ? k_rbgs_resident<2, true, false> : k_rbgs_resident<2, false, false>;
+    return ragged ? k_rbgs_resident<4, false, true> : warprow ? k_rbgs_resident<4, true, false> : k_rbgs_resident<4, false, false>;
+}
+
+cudaError_t resident_prepare(const Geom &g) {
+    Shape s;
+    if (!shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
+    return allow_smem((const void *)resident_kernel(g, s), kResSmem);
+}
+
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st) {
     Shape s;
     if (!res.work || !res.err || sweeps < 1 || !shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
     const int ctas = s.NY * s.NZ, Wq = quads_of(g);
-    const bool ragged = (g.W & 7) != 0;
     ResParams rs{s.NY, s.NZ, s.TY, s.TZ, static_cast<uint4 *>(res.work), nullptr, res.err};
     rs.epoch = reinterpret_cast<unsigned *>(rs.halo + halo_quads(g, s));
     const size_t smem = smem_of(Wq, s.TY, s.TZ);
-    const bool warprow = warp_rows(Wq, s);
-    typedef void (*Kernel)(Geom, SolveParams, const float *, const float *, float *, float *, int, ResParams);
-    const Kernel k = s.RZ == 2 ? (ragged ? k_rbgs_resident<2, false, true> : warprow ? k_rbgs_resident<2, true, false>
-                                                                                    : k_rbgs_resident<2, false, false>)
-                               : (ragged ? k_rbgs_resident<4, false, true> : warprow ? k_rbgs_resident<4, true, false>
-                                                                                    : k_rbgs_resident<4, false, false>);
-    return launch_coop(k, ctas, s.threads, smem, st, g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, rs);
+    return launch_coop(resident_kernel(g, s), ctas, s.threads, smem, st, g, sp, rhs_r, rhs_b, p_r, p_b, sweeps, rs);
 }
 
 // A batch's grids in waves of one launch each.  Every grid first gets the fewest
@@ -652,7 +648,7 @@ bool batch_resident_plan(const BatchSim *sims, int n, std::vector<ResidentWave> 
     return true;
 }
 
-void batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err) {
+cudaError_t batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err) {
     for (ResidentWave &w : *waves) {
         w.err = err;
         for (int i = 0; i < w.n; ++i) {
@@ -660,6 +656,8 @@ void batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err)
             w.grid[i].epoch = reinterpret_cast<unsigned *>(static_cast<char *>(work) + reinterpret_cast<size_t>(w.grid[i].epoch));
         }
     }
+    const cudaError_t e = allow_smem((const void *)k_batch_resident<2>, kResSmem);
+    return e != cudaSuccess ? e : allow_smem((const void *)k_batch_resident<4>, kResSmem);
 }
 
 cudaError_t launch_batch_resident(const std::vector<ResidentWave> &waves, const BatchCtl *ctl, int sweeps, cudaStream_t st) {

@@ -65,6 +65,23 @@ void launch_turb_noise(const Geom &g, const float *T, const float *U, const floa
 void launch_turb_apply(const Geom &g, float *U, float *V, float *W, const float *nU, const float *nV, const float *nW,
                        const ForceParams &fp, float *cx, float *cy, float *cz, cudaStream_t st);
 
+// A driver function through the runtime's driver entry point, null where the driver
+// has none of that name.
+template <class F> F driver_function(const char *name) {
+    void *p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return reinterpret_cast<F>(p);
+}
+// Raises a kernel's limit on dynamic shared memory, once per kernel and context.
+// The call that does so, made while this thread captures a stream and others launch,
+// can end the capture (driver 580.159), so the kernels of captured graphs are
+// prepared before (resident_prepare, advect_prepare, batch_resident_bind).
+cudaError_t allow_smem(const void *kernel, int bytes);
+
 // cuTensorMapEncodeTiled, looked up once through the runtime's driver entry
 // point (nullptr when the driver has none).
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -94,6 +111,7 @@ constexpr int kResidentVariant = kSweepVariants;
 struct ResidentWork { void *work = nullptr; int *err = nullptr; };
 bool resident_supported(const Geom &g);
 size_t resident_bytes(const Geom &g);
+cudaError_t resident_prepare(const Geom &g);
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st);
 // The temporal-blocking variant whose loads are TMA bulk copies (bounded
@@ -102,10 +120,9 @@ bool sweep_variant_uses_tma(int v);
 // Bounded TMA waits of the temporal-blocking pass that gave up since the last
 // call (then reset); nonzero means a pass produced a wrong result.
 unsigned int tb_take_timeouts();
-// Returns whether the on-chip sweeps' launch was taken (a refused one is no node of
-// a capture and leaves the capture valid; one of too many blocks for the stream's
-// context is replaced by the segment kernel); the other kernels' launch errors
-// stay for cudaGetLastError.
+// Returns whether the on-chip sweeps' launch was taken (one refused for too many
+// blocks for the stream's context is replaced by the segment kernel); the other
+// kernels' launch errors stay for cudaGetLastError.
 cudaError_t launch_rbgs_sweeps(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                                float *p_b, int sweeps, cudaStream_t st, long long *launches, int variant = 0,
                                float *q_r = nullptr, float *q_b = nullptr, const ResidentWork &res = {});
@@ -256,7 +273,7 @@ struct ResidentWave {
 };
 static_assert(sizeof(ResidentWave) <= 4000, "a wave travels as a kernel argument");
 bool batch_resident_plan(const BatchSim *sims, int n, std::vector<ResidentWave> *waves, size_t *bytes);
-void batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err);
+cudaError_t batch_resident_bind(std::vector<ResidentWave> *waves, void *work, int *err);
 cudaError_t launch_batch_resident(const std::vector<ResidentWave> &waves, const BatchCtl *ctl, int sweeps, cudaStream_t st);
 // FP64 residual of every active grid (grid s owns partial blocks
 // [blk0[s], blk0[s+1]), residual_blocks(g_s) of them) and the per-grid
@@ -334,6 +351,7 @@ int solver_warm_start(blz_solver *s, int variant, int *pre);
 int unet_timeout_flag(blz_unet *u, cudaStream_t st);
 
 // -- advection ------------------------------------------------------------------
+cudaError_t advect_prepare(const Geom &g, int scheme, bool dens);
 // D/Dn: the density scalar and its advected copy (null when not carried).
 void launch_advect(const Geom &g, const float *T, const float *U, const float *V, const float *W,
                    float *Tn, float *Un, float *Vn, float *Wn, cudaStream_t st, int scheme,

@@ -248,7 +248,8 @@ int blz_create(const blz_params *p, blz_solver **out) {
     const size_t work_at = (6 * nT + 63) / 64 * 64;
     const bool on_chip = p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 &&
                          (p->sweep_variant < 0 || p->sweep_variant == kResidentVariant) && resident_supported(g);
-    if (ok && on_chip && alloc(&s->scratch, work_at + resident_bytes(g) / sizeof(float))) {
+    if (ok && advect_prepare(g, p->advect_scheme, p->density_field != 0) != cudaSuccess) cudaGetLastError();   // its launch will tell
+    if (ok && on_chip && resident_prepare(g) == cudaSuccess && alloc(&s->scratch, work_at + resident_bytes(g) / sizeof(float))) {
         s->res.work = s->scratch + work_at;
     } else if (ok) {
         if (on_chip) cudaGetLastError();

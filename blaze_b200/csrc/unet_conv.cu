@@ -591,7 +591,7 @@ template <int N, int CIN, bool RELU>
 static cudaError_t launch_zm(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
                              void *y, const __nv_bfloat16 *aux, int *err, cudaStream_t st) {
     typedef Zm<N, CIN> Z;
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_zm<N, CIN, RELU>, cudaFuncAttributeMaxDynamicSharedMemorySize, Z::kSmem);
+    cudaError_t e = allow_smem((const void *)k_conv3d_zm<N, CIN, RELU>, Z::kSmem);
     if (e != cudaSuccess) return e;
     CUtensorMap xm;
     if (!zm_tensor_map(&xm, x, cd)) return cudaErrorNotSupported;
@@ -644,7 +644,7 @@ template <int N, bool RELU, bool F32>
 static cudaError_t launch_n(const ConvDesc &cd, const __nv_bfloat16 *x, const __nv_bfloat16 *w, const float *bias,
                             void *y, const __nv_bfloat16 *aux, int *err, cudaStream_t st) {
     const int smem = conv3d_smem_bytes(N);
-    cudaError_t e = cudaFuncSetAttribute(k_conv3d_tc<N, RELU, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void *)k_conv3d_tc<N, RELU, F32>, smem);
     if (e != cudaSuccess) return e;
     const long long interior = (long long)(cd.W + 2) * cd.H;
     const dim3 grid((unsigned)((interior + kConvM - 1) / kConvM), (unsigned)cd.D);
@@ -859,7 +859,7 @@ template <int CIN, int COUT>
 static cudaError_t launch_up_tc(int W, int H, int D, const __nv_bfloat16 *x, const __nv_bfloat16 *w,
                                 const float *bias, __nv_bfloat16 *y, int ys, int *err, cudaStream_t st) {
     typedef UpShape<CIN, COUT> S;
-    cudaError_t e = cudaFuncSetAttribute(k_upconv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
+    cudaError_t e = allow_smem((const void *)k_upconv_tc<CIN, COUT>, S::SMEM);
     if (e != cudaSuccess) return e;
     const long long tiles = ((long long)(W + 2) * H + kConvM - 1) / kConvM * D;
     const long long room = (long long)conv_sm_count() * S::kPerSm;
@@ -1027,8 +1027,7 @@ template <int CIN, int COUT>
 static cudaError_t launch_up_dgrad(int W, int H, int D, const __nv_bfloat16 *gy, int gs, const __nv_bfloat16 *w,
                                    const __nv_bfloat16 *act, __nv_bfloat16 *gx, int *err, cudaStream_t st) {
     constexpr int smem = UpDgradShape<CIN, COUT>::SMEM;
-    cudaError_t e = cudaFuncSetAttribute(k_upconv_dgrad_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         smem);
+    cudaError_t e = allow_smem((const void *)k_upconv_dgrad_tc<CIN, COUT>, smem);
     if (e != cudaSuccess) return e;
     const long long interior = (long long)(W + 2) * H;
     const dim3 grid((unsigned)((interior + kConvM - 1) / kConvM), (unsigned)D);
@@ -1273,7 +1272,7 @@ template <int MODE, int CIN, int CO>
 static cudaError_t launch_wg_tc(WgTcArgs a, cudaStream_t st) {
     using S = WgShape<MODE, CIN, CO>;
     constexpr int smem = 2 * S::BUF;
-    cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<MODE, CIN, CO>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaError_t e = allow_smem((const void *)k_wgrad_tc<MODE, CIN, CO>, smem);
     if (e != cudaSuccess) return e;
     const long long Wp = a.W + 2, plane = Wp * (a.H + 2);
     a.pbeg = plane + Wp;                                  // first interior row

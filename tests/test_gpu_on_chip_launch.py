@@ -347,3 +347,21 @@ def test_solves_at_once():
         with make(d, variant=0, **kw) as s:
             assert [s.solve()["iterations"] for _ in range(4)] == n, d
             np.testing.assert_array_equal(s.get("P"), p)
+
+
+def test_solvers_are_made_and_solved_from_several_threads():
+    """Solvers of different sizes, made, solved as device loops and closed in four
+    threads over and over: every solve graph is captured while other threads
+    allocate, launch and capture, and none of the captures ends early."""
+    dims = [(128, 128, 128), (96, 96, 96), (130, 64, 64), (64, 64, 64)]
+
+    def job(d):
+        def rounds():
+            n = set()
+            for _ in range(25):
+                with make(d, variant=-1, tol=1e-9, maxIterSolve=40, check_every=20) as s:
+                    n.add((s.solve()["iterations"], s.solve()["iterations"]))
+            return n
+        return rounds
+
+    assert in_threads([job(d) for d in dims]) == [{(40, 40)}] * 4
