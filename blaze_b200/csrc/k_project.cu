@@ -641,16 +641,7 @@ cudaError_t allow_smem(const void *kernel, int bytes) {
 }
 
 TensorMapEncodeFn tensor_map_encoder() {
-    static TensorMapEncodeFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<TensorMapEncodeFn>(p);
-    }
+    static const auto fn = driver_function<TensorMapEncodeFn>("cuTensorMapEncodeTiled");
     return fn;
 }
 

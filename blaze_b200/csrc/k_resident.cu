@@ -57,6 +57,7 @@
 // the instruction chains between the barriers; at 128^3 half of a sweep is the
 // two updates, which take most of the shared memory's bandwidth.
 #include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 #include "gs.cuh"
@@ -450,7 +451,7 @@ struct Shape { int RZ, NY, NZ, TY, TZ, threads; };
 int quads_of(const Geom &g) { return ((g.W >> 1) + 3) >> 2; }      // quads per packed row
 
 int sm_count() {
-    static int cache[64] = {0};
+    static std::atomic<int> cache[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;

@@ -17,6 +17,7 @@
 // on: 27 MMAs of M=128 x N x K=16 read one staged block.  The halo makes
 // the zero padding of the convolution a plain memory read.
 #include <algorithm>
+#include <atomic>
 
 #include <cuda_bf16.h>
 
@@ -575,7 +576,7 @@ static bool zm_tensor_map(CUtensorMap *m, const __nv_bfloat16 *x, const ConvDesc
 }
 
 static int conv_sm_count() {
-    static int cache[64] = {0};
+    static std::atomic<int> cache[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) dev = 0;
