@@ -213,7 +213,7 @@ def unet_roofline(net, scn, solver, stream, reps=3):
     flops = unet_flops((W, H, D))
     peak, kind = _peak("bf16_tflops", 1590.0)             # burst: the forward timed on its own
     achieved = flops / (ms * 1e-3) / 1e12
-    return {"bound": "tensor", "kernel": "warm-start network forward (k_conv3d_zm / k_conv3d_tc / k_upconv_tc "
+    return {"bound": "tensor", "kernel": "warm-start network forward (k_conv3d_zm / k_upconv_tc "
                                           "on tcgen05, BF16 in, FP32 accumulate; pooling, input, norms and head "
                                           "on SIMT)",
             "ms": ms, "tflop": flops / 1e12, "achieved": achieved, "peak": peak, "peak_kind": kind,
@@ -631,6 +631,8 @@ def run_batch(args, ws, rank, local):
 
 def _batch_kernel_name(v):
     """The batch autotuner's choice as reported in the stats' sweep_variant."""
+    if v == 11:
+        return "on-chip sweeps, several grids per launch (autotuned)"
     if v > 200:
         return f"temporal blocking, two sweeps per pass, tiles of {v - 200} planes, paired-FP32 stencil (autotuned)"
     if v > 100:
