@@ -8,10 +8,11 @@
 //    (kTileGrids): a CTA copies the neighbourhood its traces can reach, 40 x 16 x
 //    16 nodes of each field for 32 x 8 x 8 nodes, into shared memory, where a
 //    sample is one index plus compile-time offsets: two thirds of the
-//    instructions.  The tile's origin is shifted by three quarters of the
-//    displacement at the CTA's centre, so that it follows a uniform flow of any
-//    speed; margins of 4 nodes cover the stages' spread and the variation of the
-//    flow across the CTA.  A sample that leaves the tile reads global memory (out
+//    instructions.  The tile's origin follows the displacement at the CTA's centre
+//    (tile_follow); margins of 4 nodes cover the stages' spread, to 12 cells a step,
+//    and the variation of the flow across the CTA.  What the tile still loses to
+//    k_advect is fast flow whose samples are far apart: a shear of 120 cells a step
+//    across 128^3 takes 1120 us (917), at 256^3 4870 (4520).  A sample that leaves the tile reads global memory (out
 //    of line).  The tile repeats the field's edge nodes beyond its sides, which
 //    is what the tricubic's clamped stencil reads, so samples have no edge cases.
 //    The last faces of each axis (i = W, j = H, k = D) have blocks of their own.
@@ -291,6 +292,18 @@ __device__ __forceinline__ void tile_node(const Tile &t, const Vel &f, const Adv
     }
 }
 
+// How far the tile's origin follows the displacement d at its centre, before it is
+// rounded: three quarters of it, between the trace's stages and its end, as long as
+// the end then stays within the margin less the tricubic's one cell; in faster flow
+// to two to three cells short of the end, whose samples are the most.  Uniform flow
+// of 16 and 25 cells a step, us: 128^3 344 and 355, 256^3 2339 and 2430 (at three
+// quarters 413 and 410, 3145 and 3148; every sample general, from global memory: 355
+// and 350, 2604 and 2586).
+__device__ __forceinline__ float tile_follow(float d) {
+    const float m = fabsf(d);
+    return copysignf(0.25f * m <= (float)(kMargin - 1) ? 0.75f * m : m - ((float)kMargin - 1.5f), d);
+}
+
 template <int SCHEME, bool DENS>
 __global__ void __launch_bounds__(kAdvThreads, 1) k_advect_tile(Geom g, AdvectArrays a, int nx, int ny, int ntiles) {
     extern __shared__ float tile_s[];
@@ -311,10 +324,10 @@ __global__ void __launch_bounds__(kAdvThreads, 1) k_advect_tile(Geom g, AdvectAr
     t.s = tile_s;
     {
         const int ci = min(i0 + kTX / 2, g.W - 1), cj = min(j0 + kTY / 2, g.H - 1), ck = min(k0 + kTZ / 2, g.D - 1);
-        // three quarters of the displacement, within the margin that keeps the
-        // origin's arithmetic in range whatever the velocity (0 for a NaN)
+        // within the bounds that keep the origin's arithmetic in range whatever the
+        // velocity (0 for a NaN)
         auto shift = [&](float v, int n) {
-            const float d = -0.75f * r * v;
+            const float d = tile_follow(-r * v);
             return d == d ? __float2int_rn(fmaxf(fminf(d, (float)n), -(float)n)) : 0;
         };
         t.ox = i0 - kMargin + shift(__ldg(a.U + ci + (g.W + 1) * (cj + g.H * ck)), g.W);
