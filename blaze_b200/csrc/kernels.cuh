@@ -40,10 +40,12 @@ constexpr int kSplatBin = 8;
 // Ints per particle of the per-field index boxes: T, U, V, W and the density
 // scalar, 6 each.
 constexpr int kSplatBoxInts = 30;
-// dens (per kept particle) and Dn: the density scalar, both null when the
-// solver does not carry it.
+// scattered (splat_scattered of the bins with particles and the entries of their
+// lists): the kernel for a few particles in each bin, same sums.  dens (per kept
+// particle) and Dn: the density scalar, both null when the solver does not carry it.
+bool splat_scattered(int bins, long long entries, int fields);
 void launch_splat_gather(const Geom &g, const float *rec8, const int *boxes, const int *bin_start,
-                         const int *bin_list, const int *active, int n_active, int nbx, int nby,
+                         const int *bin_list, const int *active, int n_active, bool scattered, int nbx, int nby,
                          float *T, float *U, float *V, float *W, cudaStream_t st, const float *dens = nullptr,
                          float *Dn = nullptr);
 

@@ -50,6 +50,7 @@ struct blz_solver {
     float *pdens = nullptr;                     // per-particle density (density_field only)
     int *boxes = nullptr, *bin_start = nullptr, *bin_list = nullptr, *active = nullptr;
     int n_parts = 0, cap_parts = 0, cap_list = 0, n_active = 0;
+    bool scattered = false;                     // a few particles in each active bin
     int nbx = 0, nby = 0, nbz = 0;
     double *partials = nullptr;
     int n_partials = 0;
@@ -423,6 +424,7 @@ static int set_particles(blz_solver *s, const float *rec8, const float *dens, in
     CK(s, cudaStreamSynchronize(s->st));
     s->n_parts = m;
     s->n_active = (int)active.size();
+    s->scattered = splat_scattered(s->n_active, total, s->P.density_field ? 5 : 4);
     return BLZ_OK;
 }
 
@@ -441,7 +443,7 @@ int blz_add_source(blz_solver *s) {
     if (!s) return fail(nullptr, BLZ_ERR_ARG, "null solver");
     if (s->n_active <= 0) return BLZ_OK;
     const int c = s->cur;
-    launch_splat_gather(s->g, s->parts, s->boxes, s->bin_start, s->bin_list, s->active, s->n_active, s->nbx,
+    launch_splat_gather(s->g, s->parts, s->boxes, s->bin_start, s->bin_list, s->active, s->n_active, s->scattered, s->nbx,
                         s->nby, s->T[c], s->U[c], s->V[c], s->W[c], s->st, s->pdens, s->Dn[c]);
     CKL(s);
     s->launches += 1;

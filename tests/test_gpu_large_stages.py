@@ -78,3 +78,28 @@ def test_defect_gradient_of_several_planes(dims, bc):
     ref.gradient()
     assert_close(gpu, ref, ("P", "U", "V", "W"), rel=2e-5, absol=2e-4)
     gpu.close()
+
+
+@pytest.mark.parametrize("dens", [0, 1])
+def test_source_of_scattered_particles(dens):
+    """A few particles in each of many bins: the kernel with one block per bin for all
+    fields.  Particles on the domain's sides and outside, radii of up to 2.5 cells,
+    several in some bins; the splat test's tolerance (test_gpu_parity.py)."""
+    from blaze_b200 import FluidSolver, Timer
+    from oracle import oracle
+    scn = scene(dims=(82, 67, 91), density_field=dens, buoyancy_alpha=0.05)
+    p = scn.to_params()
+    rng = np.random.default_rng(31)
+    rec = np.zeros((1500, 8), np.float32)
+    rec[:, :3] = rng.uniform(np.array(scn.domainBboxMin) - 0.05, np.array(scn.domainBboxMax) + 0.05, (1500, 3))
+    rec[:, 3:6] = rng.uniform(-1.0, 1.0, (1500, 3))
+    rec[:, 6] = rng.uniform(0.0, 5.0, 1500) * p.dx
+    rec[:, 7] = rng.uniform(-0.5, 2.0, 1500)
+    rec[::9, 4] = 0.0                                     # a field skipped
+    d = rng.uniform(0.0, 1.0, 1500).astype(np.float32) if dens else None
+    with FluidSolver(Timer(), scn) as gpu:
+        ref = oracle.State(p, np.float64)
+        gpu.setParticles(rec, d)
+        gpu.addSource()
+        ref.add_source(rec, density=d)
+        assert_close(gpu, ref, ("T", "U", "V", "W") + (("DENSITY",) if dens else ()), rel=1e-5, absol=1e-4)
