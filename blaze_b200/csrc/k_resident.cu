@@ -561,10 +561,15 @@ static ResidentKernel resident_kernel(const Geom &g, const Shape &s) {
     return ragged ? k_rbgs_resident<4, false, true> : warprow ? k_rbgs_resident<4, true, false> : k_rbgs_resident<4, false, false>;
 }
 
-cudaError_t resident_prepare(const Geom &g) {
+cudaError_t resident_prepare(const Geom &g, int *sms) {
     Shape s;
     if (!shape_of(g, sm_count(), 0, &s)) return cudaErrorInvalidValue;
-    return allow_smem((const void *)resident_kernel(g, s), kResSmem);
+    const ResidentKernel k = resident_kernel(g, s);
+    cudaError_t e = allow_smem((const void *)k, kResSmem);
+    int per_sm = 0;
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, s.threads, smem_of(quads_of(g), s.TY, s.TZ));
+    *sms = per_sm > 0 ? (s.NY * s.NZ + per_sm - 1) / per_sm : 0;
+    return e == cudaSuccess && per_sm == 0 ? cudaErrorInvalidValue : e;
 }
 
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,

@@ -113,7 +113,7 @@ constexpr int kResidentVariant = kSweepVariants;
 struct ResidentWork { void *work = nullptr; int *err = nullptr; };
 bool resident_supported(const Geom &g);
 size_t resident_bytes(const Geom &g);
-cudaError_t resident_prepare(const Geom &g);
+cudaError_t resident_prepare(const Geom &g, int *sms);   // sms: that one launch fills
 cudaError_t launch_resident(const Geom &g, const SolveParams &sp, const float *rhs_r, const float *rhs_b, float *p_r,
                             float *p_b, int sweeps, const ResidentWork &res, cudaStream_t st);
 // The temporal-blocking variant whose loads are TMA bulk copies (bounded

@@ -6,6 +6,7 @@
 // stream (library owned unless the caller sets one).  Errors are returned as
 // BLZ_ERR_* codes with a message; nothing here exits the process.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -59,15 +60,17 @@ struct blz_solver {
     long long launches = 0;
     blz_unet *warm = nullptr;                   // learned warm start (caller owned)
     int variant = -2;                           // sweep launch shape (-2: not chosen yet)
+    int on_chip_sms = 0;                        // SMs that a launch of the on-chip sweeps fills
     ResidentWork res;                           // on-chip sweeps: exchange buffers (behind scratch; null: never chosen), error flag
     // device-loop solve: instantiated graphs (one per check interval used)
     // and their control block
+    bool crowded = false;                       // the solve in progress leaves the on-chip sweeps to others (in_use)
     struct SolveGraph {
-        int chunk = 0;
+        int chunk = 0, variant = 0;
         cudaGraphExec_t exec = nullptr;
         int body = 0, prologue = 0;
     };
-    SolveGraph graphs[8];
+    SolveGraph graphs[16];
     SolveCtl *ctl = nullptr, *h_ctl = nullptr;
     // automatic check interval (check_every < 0): the last solve's sweeps and
     // its measured cost of one residual check in sweeps
@@ -250,7 +253,7 @@ int blz_create(const blz_params *p, blz_solver **out) {
     const bool on_chip = p->gs_order == BLZ_GS_RB3D && p->temporal_block == 0 &&
                          (p->sweep_variant < 0 || p->sweep_variant == kResidentVariant) && resident_supported(g);
     if (ok && advect_prepare(g, p->advect_scheme, p->density_field != 0) != cudaSuccess) cudaGetLastError();   // its launch will tell
-    if (ok && on_chip && resident_prepare(g) == cudaSuccess && alloc(&s->scratch, work_at + resident_bytes(g) / sizeof(float))) {
+    if (ok && on_chip && resident_prepare(g, &s->on_chip_sms) == cudaSuccess && alloc(&s->scratch, work_at + resident_bytes(g) / sizeof(float))) {
         s->res.work = s->scratch + work_at;
     } else if (ok) {
         if (on_chip) cudaGetLastError();
@@ -660,6 +663,22 @@ static int take_resident_error(blz_solver *s) {
     return resident_gave_up(s) ? fail(s, BLZ_ERR_TIMEOUT, "on-chip sweeps: a bounded wait between blocks gave up") : BLZ_OK;
 }
 
+// Solves in progress, by device.  The blocks of an on-chip launch must all run at
+// once, so solves on several streams take turns with the SMs, where the segment
+// kernel's launches run beside one another: from two and a half devices' worth of
+// SMs on, a solve that tunes its sweeps takes the segment kernel (same bits).
+// us per sweep and solver with 1, 2, 4, 8 solves at once: 64^3 2.0, 1.8, 1.5, 0.9 (on
+// chip whatever the number 2.0, 1.8, 1.8, 1.8; never 4.0, 2.3, 1.4, 0.8), 120 x 100 x
+// 84 3.5, 3.3, 2.4, 2.6 (3.5, 3.4, 3.4, 3.4; 5.4, 3.4, 2.2, 2.4).
+static std::atomic<int> g_solving[64];
+struct Solving {
+    std::atomic<int> &n;
+    int at_once;
+    explicit Solving(int device) : n(g_solving[device & 63]), at_once(n.fetch_add(1) + 1) {}
+    ~Solving() { n.fetch_sub(1); }
+};
+static int in_use(const blz_solver *s) { return s->crowded && s->variant == kResidentVariant ? ((s->g.W & 7) ? -1 : 0) : s->variant; }
+
 static int choose_variant(blz_solver *s) {
     if (s->variant != -2) return BLZ_OK;
     const int nv = s->P.temporal_block == 1 ? std::min(sweep_variant_count(s->g), kSegVariants)
@@ -783,7 +802,7 @@ static int sweeps_on(blz_solver *s, int n, const float *rr, const float *rb, flo
     } else {
         int rc = choose_variant(s);
         if (rc != BLZ_OK) return rc;
-        CK(s, launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, s->variant, q_r(s), q_b(s), s->res));
+        CK(s, launch_rbgs_sweeps(s->g, sp, rr, rb, pr, pb, n, s->st, &s->launches, in_use(s), q_r(s), q_b(s), s->res));
     }
     CKL(s);
     return BLZ_OK;
@@ -823,18 +842,19 @@ static int solve_device_loop(blz_solver *s, blz_step_stats *st, int chunk) {
     if (rc != BLZ_OK) return rc;
     blz_solver::SolveGraph *gr = nullptr;
     for (auto &x : s->graphs)
-        if (x.exec && x.chunk == chunk) gr = &x;
+        if (x.exec && x.chunk == chunk && x.variant == in_use(s)) gr = &x;
     const DefectArrays dfa = defect_arrays(s);
     if (!gr) {
         for (auto &x : s->graphs)
             if (!x.exec) { gr = &x; break; }
         if (!gr) return fail(s, BLZ_ERR_STATE, "too many check intervals");
         cudaError_t e = build_solve_graph(s->g, solve_params(P), s->sr_r, s->sr_b, s->sx_r, s->sx_b, s->partials,
-                                          s->n_partials, s->d_norm2, s->ctl, chunk, P.max_iter, P.tol, s->variant,
+                                          s->n_partials, s->d_norm2, s->ctl, chunk, P.max_iter, P.tol, in_use(s),
                                           s->st, &gr->exec, &gr->body, &gr->prologue, q_r(s), q_b(s),
                                           P.defect_correction ? &dfa : nullptr, s->res);
         if (e != cudaSuccess) return fail(s, BLZ_ERR_CUDA, "building the solve graph failed: %s", cudaGetErrorString(e));
         gr->chunk = chunk;
+        gr->variant = in_use(s);
     }
     CK(s, cudaGraphLaunch(gr->exec, s->st));
     CK(s, cudaMemcpyAsync(s->h_ctl, s->ctl, sizeof(SolveCtl), cudaMemcpyDeviceToHost, s->st));
@@ -854,7 +874,7 @@ static int solve_device_loop(blz_solver *s, blz_step_stats *st, int chunk) {
         st->ms_sweeps = (float)(c.sweep_ns * 1e-6);
         st->ms_checks = (float)(c.check_ns * 1e-6);
         st->residual_checks = c.checks;
-        st->sweep_variant = s->variant;
+        st->sweep_variant = in_use(s);
         st->device_loop = 1;
         st->check_interval = chunk;
         if (!std::isfinite(r)) return fail(s, BLZ_ERR_NAN, "non-finite residual after %d sweeps", c.iters);
@@ -888,7 +908,7 @@ static int warm_start(blz_solver *s, int variant, int *pre) {
     if (*pre > 0 && P.gs_order == BLZ_GS_RB3D) {
         if (variant < 0) {
             if ((rc = sweeps(s, *pre)) != BLZ_OK) return rc;
-            variant = s->variant;
+            variant = in_use(s);
         } else {
             CK(s, launch_rbgs_sweeps(s->g, solve_params(P), s->sr_r, s->sr_b, s->sx_r, s->sx_b, *pre, s->st,
                                      &s->launches, variant, q_r(s), q_b(s)));
@@ -907,6 +927,9 @@ static int warm_start(blz_solver *s, int variant, int *pre) {
 int blz_solve(blz_solver *s, blz_step_stats *st) {
     if (!s) return fail(nullptr, BLZ_ERR_ARG, "null solver");
     const blz_params &P = s->P;
+    const Solving solving(s->device);
+    s->crowded = s->res.work && P.sweep_variant < 0 && solving.at_once > 1 &&
+                 2 * solving.at_once * s->on_chip_sms > 5 * 148;
     const size_t half = n_of(P, 0) / 2;
     if (P.reset_pressure) {
         CK(s, cudaMemsetAsync(s->p_r, 0, half * sizeof(float), s->st));
@@ -1026,7 +1049,7 @@ static int solve_body(blz_solver *s, blz_step_stats *st) {
         st->converged = P.tol <= 0.0 || b == 0.0 || r / b <= P.tol;
         st->ms_sweeps = ms_sweeps;
         st->residual_checks = checks;
-        st->sweep_variant = s->variant;
+        st->sweep_variant = in_use(s);
         st->device_loop = 0;
         st->check_interval = chunk;
         st->ms_checks = 0.0f;
@@ -1039,6 +1062,7 @@ int blz_sweeps(blz_solver *s, int n) {
     if (!s) return fail(nullptr, BLZ_ERR_ARG, "null solver");
     if (n < 0) return fail(s, BLZ_ERR_ARG, "negative sweep count %d", n);
     s->defect_valid = false;                    // p changes on its own: drop the remainder
+    s->crowded = false;
     const int rc = n > 0 ? sweeps_on(s, n, s->rhs_r, s->rhs_b, s->p_r, s->p_b) : BLZ_OK;
     return rc != BLZ_OK ? rc : check_tb_timeouts(s);
 }

@@ -365,3 +365,24 @@ def test_solvers_are_made_and_solved_from_several_threads():
         return rounds
 
     assert in_threads([job(d) for d in dims]) == [{(40, 40)}] * 4
+
+
+def test_tuned_solves_at_once_give_the_bits_of_one(monkeypatch):
+    """Eight solves at once of solvers that tune their sweeps, some of which leave the
+    on-chip sweeps to others: sweep counts and pressures are the segment kernel's."""
+    monkeypatch.delenv("BLZ_SWEEP_VARIANT", raising=False)
+    kw = dict(tol=1e-9, maxIterSolve=200, check_every=20)
+    dims = [(64, 64, 64), (26, 60, 58), (120, 50, 44), (64, 40, 72)] * 2
+
+    def job(d):
+        def solve():
+            with make(d, variant=-1, **kw) as s:
+                st = [s.solve() for _ in range(6)]
+                assert all(x["sweep_variant"] in (0, -1, 4, ON_CHIP) for x in st), st
+                return [x["iterations"] for x in st], s.get("P")
+        return solve
+
+    for d, (n, p) in zip(dims, in_threads([job(d) for d in dims])):
+        with make(d, variant=0, **kw) as s:
+            assert [s.solve()["iterations"] for _ in range(6)] == n, d
+            np.testing.assert_array_equal(s.get("P"), p)
