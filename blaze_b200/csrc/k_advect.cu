@@ -10,11 +10,12 @@
 //    sample is one index plus compile-time offsets: two thirds of the
 //    instructions.  The tile's origin follows the displacement at the CTA's centre
 //    (tile_follow); margins of 4 nodes cover the stages' spread, to 12 cells a step,
-//    and the variation of the flow across the CTA.  What the tile still loses to
-//    k_advect is fast flow whose samples are far apart: a shear of 120 cells a step
-//    across 128^3 takes 1120 us (917), at 256^3 4870 (4520).  A sample that leaves the tile reads global memory (out
-//    of line).  The tile repeats the field's edge nodes beyond its sides, which
-//    is what the tricubic's clamped stencil reads, so samples have no edge cases.
+//    and the variation of the flow across the CTA.  A sample that leaves the tile
+//    reads global memory (out of line).  What the tile loses to k_advect is fast
+//    flow whose samples are far apart: a shear of 120 cells a step across 128^3
+//    takes 1120 us (917), at 256^3 4870 (4520).  The tile repeats the field's edge
+//    nodes beyond its sides, which is what the tricubic's clamped stencil reads, so
+//    samples have no edge cases.
 //    The last faces of each axis (i = W, j = H, k = D) have blocks of their own.
 //  - k_advect, a thread per node and all four fields, from global memory: on a
 //    small grid one wave of 1024-thread CTAs that first copy a tile waits longer.

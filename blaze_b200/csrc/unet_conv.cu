@@ -238,8 +238,9 @@ k_conv3d_tc(int W, int H, int D, int cin, int out_stride, int out_offset, const 
 int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 
 // ---------------------------------------------------------------------------
-// z-marching variant for the layers of 16 to 128 input and output channels.  A CTA keeps the layer's weights resident and walks a tile of 8 x 16
-// voxels (x, y) through `zs` output planes.
+// z-marching variant for the layers of 16 to 128 input and output channels.  A
+// CTA keeps the layer's weights resident and walks a tile of 8 x 16 voxels (x, y)
+// through `zs` output planes.
 //
 // What bounds such a layer is the number of MMAs: with 16 output channels one
 // of 128 x 16 x 16 takes as long as one three times as wide, since both read the
@@ -277,9 +278,9 @@ int conv3d_smem_bytes(int cout) { return kABytes + 27 * cout * 32; }
 // 81 and 252 (general kernel about 228 and 456).  What bounds it is the MMA warp: a block
 // costs it about 900 cycles of waits, descriptors and 9 or 10 MMAs, with the
 // copies taken out as with them.  So small layers share an SM, up to four CTAs
-// (16 -> 16: 460 us with two), where the MMAs' operands then take the shared
-// memory's bandwidth (48 cycles an MMA; 44 for 4 KB of voxels and 1.5 KB of
-// weights); the usual case of three planes inside the ring has its own path with
+// (16 -> 16: 460 us with two; at 192^3 an SM then issues an MMA every 66 cycles,
+// the tensor pipe is active 34 % of the time and the fullest unit is the L1, 77 %);
+// the usual case of three planes inside the ring has its own path with
 // constant descriptors, and an elected lane issues (64 -> 32: 360 us without the
 // two).  The swizzle's 32-byte runs against 16-byte ones: 343 against 367 (16 ->
 // 16, before the last two).

@@ -115,7 +115,8 @@ typedef struct blz_params {
                                      reference keeps p between frames)      */
     int    max_particles;         /* sourceMaxParticleCount                  */
     int    temporal_block;        /* 0: the autotuner may pick the two-sweeps-
-                                     per-HBM-pass kernel; 1: unblocked
+                                     per-HBM-pass kernel, or the on-chip
+                                     sweeps where the grid fits; 1: unblocked
                                      sweeps only                             */
     int    device_loop;           /* 1: a residual-controlled solve runs as one
                                      CUDA graph whose conditional WHILE node
@@ -123,7 +124,13 @@ typedef struct blz_params {
                                      trip per check); needs max_iter to be a
                                      multiple of check_every                 */
     int    sweep_variant;         /* -1: autotune the sweep launch shape per
-                                     grid size (first solve); >= 0: force one */
+                                     grid size (first solve); >= 0: force one
+                                     (11: the on-chip sweeps, where the grid
+                                     fits, up to about 2 million cells).
+                                     Tuned solves in progress at once beyond
+                                     what the SMs hold of on-chip launches
+                                     take the segment kernel; every choice
+                                     gives the same bits                     */
     int    advect_scheme;         /* BLZ_ADVECT_*: backtrace integrator       */
     /* Target mode only (no counterpart in the reference, whose buoyancy is
      * beta * T alone, FluidSolver.cu:142-156): a smoke density scalar on the
@@ -491,14 +498,16 @@ int  blz_batch_create(blz_solver *const *solvers, int n, blz_batch **out);
 int  blz_batch_destroy(blz_batch *b);
 void *blz_batch_stream(blz_batch *b);                      /* the batch's cudaStream_t */
 /* Sweep kernel of the batched solve: planes = -1 (default) autotunes between
- * the segment kernel (one sweep per pass over HBM) and temporal blocking (two
+ * the segment kernel (one sweep per pass over HBM), temporal blocking (two
  * sweeps per pass, tiles of 8, 16 or 32 planes, scalar or paired-FP32
- * stencil); 0 forces the segment kernel; planes > 0 forces temporal blocking
+ * stencil) and, where every grid fits, the on-chip sweeps of several grids
+ * side by side; 0 forces the segment kernel; planes > 0 forces temporal blocking
  * with tiles of that many planes, paired != 0 with the paired-FP32 stencil
  * (BLZ_ERR_ARG unless check_every % 4 == 0 and every grid has width % 8 == 0
  * and width <= 384).  Every choice gives the same bits.  The stats'
  * sweep_variant reports the choice: the segment kernel's planes per thread
- * (1, 2, 4, 8), or 100 (scalar) or 200 (paired) + planes per tile.         */
+ * (1, 2, 4, 8), 100 (scalar) or 200 (paired) + planes per tile, or 11 (on
+ * chip).                                                                    */
 int  blz_batch_set_sweep(blz_batch *b, int planes, int paired);
 int  blz_batch_add_source(blz_batch *b);                   /* blz_add_source of every solver */
 /* One frame of every solver: forces at times[i] (NULL: 0), divergence, the
